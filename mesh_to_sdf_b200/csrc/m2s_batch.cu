@@ -87,7 +87,7 @@ uint64_t tune_key(const GridJob& job) {
   cudaGetDevice(&dev);
   uint64_t lg = 0;
   while ((1ull << lg) < job.cells()) ++lg;
-  return ((uint64_t)dev << 32) | ((uint64_t)job.sign() << 16) | ((uint64_t)(job.grids() > 1) << 8) | lg;
+  return ((uint64_t)dev << 32) | ((uint64_t)(job.threads() / 256) << 24) | ((uint64_t)job.sign() << 16) | ((uint64_t)(job.grids() > 1) << 8) | lg;
 }
 
 }  // namespace

@@ -699,7 +699,7 @@ __global__ void k_barrier_probe(GridBarrier* bar, unsigned int expected, unsigne
 // Touched cells staged per block and round in shared memory; a block commits
 // the cells it touched itself, so only a block whose stage fills up writes to
 // the global spill list.
-constexpr int kTouchStage = 6144;
+constexpr uint32_t kStagePerThread = 24;  // stage entries per thread of the block
 constexpr int kUnroll = 2;  // proposals per thread in flight
 
 
@@ -780,14 +780,25 @@ struct WarpQueue {
   float px[kQueue], py[kQueue], pz[kQueue];  // the neighbour's cell centre
   unsigned long long snap[kQueue];
 };
-constexpr int kWarps = 8;  // k_propagate runs 256 threads per block
+// k_propagate's block sizes.  An SM holds 1,024 of its threads (64 registers
+// each) as one, two or four blocks.  Fewer blocks are fewer arrivals at a grid
+// barrier and fewer adds to the list counters, more blocks wait less for their
+// slowest warp at block barriers (256 / 512 / 1,024 threads: 32^3 462 / 482 /
+// 515 us, 97 x 110 x 75 2,244 / 2,164 / 2,213, 24 grids of 32M cells 23.2 /
+// 21.7 / 22.2 ms, 256^3 8.69 / 8.48 / 8.32 ms).  The lines lie at the powers
+// of two that bound the autotuner's classes.  blocks_per_sm counts blocks of
+// 256, and the filtered kernel (80 registers) runs three of those per SM.
+constexpr uint32_t kSmallBlock = 256, kBigBlock = 1024;
+inline uint32_t block_threads(unsigned long long cells) {
+  return cells <= 1ull << 18 ? kSmallBlock : (cells <= 1ull << 23 ? 512u : kBigBlock);
+}
 
 // Stages cell j, whose first lowering of the round this proposal made, for the
 // block's commit (spilling to the round's global list when the stage is full).
 __device__ __forceinline__ void stage_touch(uint32_t j, uint32_t* s_touch, uint32_t* s_ntouch, PropState* st,
                                             uint32_t parity, uint32_t* spill, uint32_t cap) {
   const uint32_t q = atomicAdd(s_ntouch, 1u);
-  if (q < kTouchStage) {
+  if (q < kStagePerThread * blockDim.x) {
     s_touch[q] = j;
   } else {
     const uint32_t pos = atomicAdd(&st->touched2[parity], 1u);
@@ -843,7 +854,7 @@ __device__ __forceinline__ bool propose_at(const TriRec& r, uint32_t tri, uint32
 constexpr uint32_t kHash = 2048;
 constexpr uint32_t kNoCell = 0xFFFFFFFFu;
 static_assert(26 * kSoloCap < kHash, "a solo round could fill the table");
-static_assert(kHash * 3 <= (uint32_t)kTouchStage, "the table exceeds the touch stage");
+static_assert(kHash * 3 <= kStagePerThread * kSmallBlock, "the table exceeds the touch stage");
 
 __device__ __forceinline__ uint32_t hash_slot(uint32_t j) { return (j * 2654435761u) >> 21; }  // 11 bits
 
@@ -1246,7 +1257,7 @@ __device__ __forceinline__ void relax_commit(const GridSet& gs, unsigned long lo
 // 4 blocks of 256 threads fit per SM (64 registers a thread); the filtered
 // propose loop needs about 80 registers, so that variant runs 3 per SM.
 template <int SIGN, bool MULTI, bool FILTER>
-__global__ void __launch_bounds__(256, FILTER ? 3 : 4) k_propagate(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris,
+__global__ void __launch_bounds__(FILTER ? kSmallBlock : kBigBlock, FILTER ? 3 : 1) k_propagate(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris,
                                                    unsigned long long* keys,
                                                    uint2* lists, uint32_t cap, uint32_t* spill_lists,
                                                    PropState* st, GridBarrier* bar, uint32_t max_steps,
@@ -1254,10 +1265,11 @@ __global__ void __launch_bounds__(256, FILTER ? 3 : 4) k_propagate(const __grid_
                                                    uint32_t solo_max, const TriBound* __restrict__ bounds,
                                                    const float* __restrict__ slack) {
   __shared__ Sched sh;
-  __shared__ __align__(16) uint32_t s_touch[kTouchStage];  // also a solo run's min table
+  // [cells touched this round (also a solo run's min table) | the warps' queues]
+  extern __shared__ __align__(16) uint32_t s_touch[];
   __shared__ uint16_t s_taken[26 * kSoloCap];              // a solo round's taken table slots
   constexpr bool kQueued = SIGN == M2S_SIGN_NORMAL || FILTER;  // the plain Raycast loop needs no queue
-  __shared__ WarpQueue s_queue[kQueued ? kWarps : 1];
+  WarpQueue* s_queue = reinterpret_cast<WarpQueue*>(s_touch + kStagePerThread * blockDim.x);
   __shared__ uint32_t s_ntouch, s_gen, s_pending, s_more, s_runs, s_solo_run;
   __shared__ uint32_t s_count[kLists], s_far_min[2], s_overflow;  // block 0's counters during a solo run
   // (built where used, so no pointer stays live across the propose loop)
@@ -1450,7 +1462,7 @@ __global__ void __launch_bounds__(256, FILTER ? 3 : 4) k_propagate(const __grid_
     } else {
       if (lead_block && threadIdx.x == 0) st->touched2[parity ^ 1u] = 0;
       const uint32_t nspill = min(*(volatile uint32_t*)&st->touched2[parity], cap);
-      relax_commit<MULTI>(gs, keys, s_touch, min(s_ntouch, (uint32_t)kTouchStage), spill, nspill, t0,
+      relax_commit<MULTI>(gs, keys, s_touch, min(s_ntouch, kStagePerThread * blockDim.x), spill, nspill, t0,
                           T, st, sh, lists, cap, &s_push, push_turn);
     }
     if (!solo) {
@@ -1736,10 +1748,23 @@ PropState* host_state() {
   return h.p;
 }
 
+size_t propagate_smem(uint32_t threads, int sign, bool filter) {
+  return threads * kStagePerThread * sizeof(uint32_t) +
+         (sign == M2S_SIGN_NORMAL || filter ? threads / 32 * sizeof(WarpQueue) : 0);
+}
 template <int SIGN>
 const void* propagate_kernel(bool multi, bool filter) {
   if (filter) return multi ? (const void*)k_propagate<SIGN, true, true> : (const void*)k_propagate<SIGN, false, true>;
   return multi ? (const void*)k_propagate<SIGN, true, false> : (const void*)k_propagate<SIGN, false, false>;
+}
+
+// Blocks of the propagation kernel that fit on one SM.
+cudaError_t propagate_fit(const void* kern, uint32_t threads, int sign, bool filter, int* per_sm) {
+  const size_t smem = propagate_smem(threads, sign, filter);
+  // (more shared memory than a kernel gets without asking)
+  const size_t most = propagate_smem(filter ? kSmallBlock : kBigBlock, sign, filter);
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, (int)threads, smem);
 }
 
 }  // namespace
@@ -1756,6 +1781,7 @@ struct GridJob::Impl {
   uint32_t cap = 0;
   unsigned coop_blocks = 0;
   unsigned coop_max = 0;
+  uint32_t threads = kSmallBlock;
   uint32_t solo_max = 64;
   unsigned long long ray_words = 0;
   uint64_t launches = 0;
@@ -1796,6 +1822,7 @@ unsigned GridJob::max_cooperative_blocks() const { return p->coop_max; }
 void GridJob::set_cooperative_blocks(unsigned blocks) { p->coop_blocks = std::max(1u, std::min(blocks, p->coop_max)); }
 int GridJob::sign() const { return p->sign; }
 uint32_t GridJob::grids() const { return p->gs.ngrids; }
+uint32_t GridJob::threads() const { return p->threads; }
 uint64_t GridJob::device_bytes() const {
   const Impl& J = *p;
   return J.comb_tris.n * sizeof(TriRec) + J.tri_grid.n * 4 + J.keys.n * 8 + J.bits.n * 4 +
@@ -1808,7 +1835,7 @@ int propagate_blocks_per_sm(int sign) {
   const void* kern = sign == M2S_SIGN_RAYCAST ? propagate_kernel<M2S_SIGN_RAYCAST>(true, filter)
                                               : propagate_kernel<M2S_SIGN_NORMAL>(true, filter);
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) != cudaSuccess) return 1;
+  if (propagate_fit(kern, kSmallBlock, sign, filter, &per_sm) != cudaSuccess) return 1;
   return std::max(per_sm, 1);
 }
 
@@ -1939,7 +1966,8 @@ int GridJob::prepare(const MeshView* meshes, uint32_t n, const GridDesc* gds, in
   int dev = 0, sms = 0, per_sm = 0;
   M2S_CUDA(cudaGetDevice(&dev));
   M2S_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  M2S_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0));
+  J.threads = J.filter || tune.blocks_per_sm > 0 ? kSmallBlock : block_threads(N);
+  M2S_CUDA(propagate_fit(kern, J.threads, sign, J.filter, &per_sm));
   if (per_sm < 1) {
     set_error("grid propagation kernel cannot be resident");
     return M2S_ERR_CUDA;
@@ -2013,8 +2041,8 @@ int GridJob::enqueue(cudaStream_t s, cudaEvent_t* ev) {
                     &J.bounds.p, &J.slack.p};
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(J.coop_blocks);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = 0;
+    cfg.blockDim = dim3(J.threads);
+    cfg.dynamicSmemBytes = propagate_smem(J.threads, J.sign, J.filter);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

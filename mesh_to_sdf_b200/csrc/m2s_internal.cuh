@@ -252,6 +252,7 @@ class GridJob {
   void set_cooperative_blocks(unsigned blocks);  // clamped to [1, max_cooperative_blocks()]
   int sign() const;
   uint32_t grids() const;
+  uint32_t threads() const;  // of a propagation block
   // Profiling: record every propagation step (kind and size, and the time it
   // was chosen) in a device log of `cap` steps.
   int enable_round_log(uint32_t cap, cudaStream_t s);
