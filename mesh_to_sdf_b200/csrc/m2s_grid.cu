@@ -42,10 +42,12 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstddef>
 #include <cmath>
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "m2s_audit.cuh"
@@ -171,6 +173,11 @@ struct Sched {
   int action;
 };
 
+constexpr uint32_t kParts = 32;
+enum { kCountSeeds, kCountRayHits, kCountEvals, kCountSame, kCountBound, kCounts };
+struct __align__(128) CountPart {
+  unsigned long long n;
+};
 struct PropState {
   Sched handoff;         // the schedule block 0 leaves after relaxing rounds alone
   uint32_t b;            // current bucket
@@ -190,13 +197,24 @@ struct PropState {
   uint32_t log_n;         // steps recorded in the round log
   uint32_t solo_rounds;   // rounds relaxed by block 0 alone
   unsigned long long entries, evals, seeds, ray_hits;
+  uint32_t big_seeds, big_rays;  // chunks of large triangles left to k_seed_chunks / k_ray_chunks
   unsigned long long filter_same;   // proposals dropped: the neighbour holds the proposing triangle
   unsigned long long filter_bound;  // proposals dropped by the distance bound
   // FP64 audit (GridTuning::fp64_audit): ray tests, ambiguous, FP64 decides
   // otherwise; cells whose 2-of-3 vote the FP64 decisions flip; cells whose
   // region was audited (proper triangles), ambiguous, FP64 picks another.
   unsigned long long audit[kAuditStats];
+  // Counts that every warp adds to, as kParts parts a cache line apart: one
+  // word takes its atomics one after another, about 1 ns each (256^3 grid,
+  // 81,920 triangles: rays 138 -> 90 us, seeding 96 -> 83 us).  k_finalize sums
+  // them into the words above; the host does not read them.
+  CountPart parts[kCounts][kParts];
 };
+
+__device__ __forceinline__ void add_count(PropState* st, int which, unsigned long long n) {
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  atomicAdd(&st->parts[which][warp % kParts].n, n);
+}
 
 __device__ __forceinline__ P3 center(const GridK& g, int x, int y, int z) {
   // grid.rs:135-141: first + (i as f32) * size
@@ -373,12 +391,6 @@ __device__ __forceinline__ bool bound_rejects(const TriBound& tb, float sl, P3 p
   return lb2 > thr * thr;                     // false when thr is infinite or anything is NaN
 }
 
-__global__ void k_fill_u64(unsigned long long* p, unsigned long long n, unsigned long long v) {
-  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (unsigned long long)gridDim.x * blockDim.x)
-    p[i] = v;
-}
-
 // Batch triangle array: triangle t of the job is triangle t - tri_off[k] of
 // mesh k.  Keys store the job-wide index, which keeps each mesh's triangle
 // order, so ties resolve exactly as for the mesh alone.
@@ -392,20 +404,71 @@ __global__ void k_gather_tris(const TriRec* const* __restrict__ src, const uint3
   }
 }
 
+constexpr unsigned int kMaxBarrierBlocks = 2048;
+// (how it works: at grid_barrier)
+struct GridBarrier {
+  unsigned int arrivals;
+  unsigned int abort;
+  unsigned int pad0[30];
+};
+
 // ---- 1. seeding -------------------------------------------------------------
-template <int SIGN, bool MULTI>
-__global__ void k_seed(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t T,
-                       unsigned long long* keys, uint32_t* status, PropState* st) {
-  const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= T) return;
-  const GridK& g = grid_of_tri<MULTI>(gs, t);
-  TriRec r = tris[t];
-  P3 a = p3(r.a), b = p3(r.b), c = p3(r.c);
-  int kind = __float_as_int(r.a.w);
+// Everything a run starts from, in one launch (the memsets and small kernels it
+// replaces were four launches more): empty keys, the state, the barrier and
+// the ray bits (bits64: the FP64 audit's, may be NULL).
+__global__ void k_init(ulonglong2* keys2, unsigned long long ncell, PropState* st, GridBarrier* bar, uint32_t* bits,
+                       uint32_t* bits64, unsigned long long words) {
+  const unsigned long long i0 = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  for (unsigned long long i = i0; i < ncell / 2; i += stride) keys2[i] = make_ulonglong2(KEY_EMPTY, KEY_EMPTY);
+  if (i0 == 0 && (ncell & 1u)) reinterpret_cast<unsigned long long*>(keys2)[ncell - 1] = KEY_EMPTY;
+  for (unsigned long long i = i0; i < words; i += stride) {
+    bits[i] = 0u;
+    if (bits64) bits64[i] = 0u;
+  }
+  if (blockIdx.x == 0) {
+    for (uint32_t w = threadIdx.x; w < sizeof(PropState) / 4; w += blockDim.x) reinterpret_cast<uint32_t*>(st)[w] = 0u;
+    for (uint32_t w = threadIdx.x; w < sizeof(GridBarrier) / 4; w += blockDim.x)
+      reinterpret_cast<uint32_t*>(bar)[w] = 0u;
+    __syncthreads();
+    if (threadIdx.x < kRing) st->slot[threadIdx.x] = threadIdx.x;
+    if (threadIdx.x == 0) {
+      st->cur = kCur0;
+      st->far_min[0] = st->far_min[1] = kNoBucket;
+    }
+  }
+}
+
+// Seeding and rays give a triangle to one warp, which is right while its box
+// holds about as many cells as the warp has lanes.  The box of a large one (a
+// coarse mesh in a fine grid; the long windows that join a strip's rows) would
+// keep its warp busy long after the others have left (the terrain strip's
+// seeding: 1.62 ms, 0.60 + 0.12 ms with the split), so a box of more than kSplitCells cells is left in
+// chunks of kChunkCells for a second kernel, a warp each.  The list holds
+// kMaxChunks; a triangle that does not fit stays with its warp.
+constexpr uint32_t kSplitCells = 1024, kChunkCells = 512, kMaxChunks = 1u << 18;
+constexpr uint32_t kNoChunk = 0xFFFFFFFFu;
+// Lists the chunks of triangle t (each as (t, first + chunk * step)) and
+// returns true, or returns false: the caller does the whole box.  All 32 lanes call it.
+__device__ __forceinline__ bool split_box(uint32_t t, unsigned long long total, uint32_t first, uint32_t step,
+                                          uint32_t* count, uint2* chunks) {
+  if (total <= kSplitCells || total > (unsigned long long)kMaxChunks * kChunkCells) return false;
+  const uint32_t lane = threadIdx.x & 31u, nch = (uint32_t)((total + kChunkCells - 1) / kChunkCells);
+  // (Once the list is full nobody adds: the counter cannot wrap.)
+  uint32_t base = kMaxChunks;
+  if (lane == 0 && *(volatile uint32_t*)count < kMaxChunks) base = atomicAdd(count, nch);
+  base = __shfl_sync(0xFFFFFFFFu, base, 0);
+  const bool fits = base < kMaxChunks && nch <= kMaxChunks - base;
+  for (uint32_t k = lane; k < nch && base < kMaxChunks && base + k < kMaxChunks; k += 32u)
+    chunks[base + k] = make_uint2(fits ? t : kNoChunk, first + k * step);
+  return fits;
+}
+
+// The box of cells that triangle r seeds (grid.rs:400-426).
+__device__ __forceinline__ void seed_box(const GridK& g, const TriRec& r, int mn[3], int ext[3]) {
   P3 lo, hi;
-  padded_box(a, b, c, &lo, &hi);  // grid.rs:400
-  int mn[3], mx[3];
+  padded_box(p3(r.a), p3(r.b), p3(r.c), &lo, &hi);  // grid.rs:400
+  int mx[3];
   snap(g, lo, mn);
   snap(g, hi, mx);
   // grid.rs:410-426: widen by one cell where the box pokes past a centre.
@@ -414,10 +477,18 @@ __global__ void k_seed(const __grid_constant__ GridSet gs, const TriRec* __restr
   for (int d = 0; d < 3; ++d) {
     if (mn[d] > 0 && vget(mnf, d) > vget(lo, d)) mn[d] -= 1;
     if (mx[d] < g.n[d] - 1 && vget(mxf, d) < vget(hi, d)) mx[d] += 1;
+    ext[d] = mx[d] - mn[d] + 1;
   }
-  long long ex = mx[0] - mn[0] + 1, ey = mx[1] - mn[1] + 1, ez = mx[2] - mn[2] + 1;
-  if (ex <= 0 || ey <= 0 || ez <= 0) return;
-  long long total = ex * ey * ez;
+}
+
+// Triangle t at cells k0 <= k < k1 of its box (z fastest), on one warp.
+template <int SIGN>
+__device__ __forceinline__ void seed_cells(const GridK& g, const TriRec& r, uint32_t t, const int mn[3],
+                                           const int ext[3], unsigned long long k0, unsigned long long k1,
+                                           unsigned long long* keys, uint32_t* status, PropState* st) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const P3 a = p3(r.a), b = p3(r.b), c = p3(r.c);
+  const int kind = __float_as_int(r.a.w);
   bool nan = false;
   uint32_t updates = 0;
   auto visit = [&](int x, int y, int z) {
@@ -425,19 +496,54 @@ __global__ void k_seed(const __grid_constant__ GridSet gs, const TriRec* __restr
     if (isnan(d)) nan = true;
     if (update_min<SIGN>(&keys[g.cell_off + local_index(g, x, y, z)], pack(d, t), &nan)) ++updates;
   };
-  if (total <= 0x7FFFFFFFll) {  // 32-bit division (64-bit costs ~4x the instructions)
-    const uint32_t uez = (uint32_t)ez, uey = (uint32_t)ey, utotal = (uint32_t)total;
-    for (uint32_t k = lane; k < utotal; k += 32) {
+  const uint32_t uey = (uint32_t)ext[1], uez = (uint32_t)ext[2];
+  if (k1 <= 0x7FFFFFFFull) {  // 32-bit division (64-bit costs ~4x the instructions)
+    for (uint32_t k = (uint32_t)k0 + lane; k < (uint32_t)k1; k += 32) {
       const uint32_t q = k / uez, xq = q / uey;
       visit(mn[0] + (int)xq, mn[1] + (int)(q - xq * uey), mn[2] + (int)(k - q * uez));
     }
   } else {
-    for (long long k = lane; k < total; k += 32)
-      visit(mn[0] + (int)(k / (ez * ey)), mn[1] + (int)((k / ez) % ey), mn[2] + (int)(k % ez));
+    for (unsigned long long k = k0 + lane; k < k1; k += 32) {
+      const unsigned long long q = k / uez;
+      visit(mn[0] + (int)(q / uey), mn[1] + (int)(q % uey), mn[2] + (int)(k % uez));
+    }
   }
   if (nan) atomicOr(status, bit(M2S_ERR_NAN_DISTANCE));
   for (int o = 16; o; o >>= 1) updates += __shfl_xor_sync(0xFFFFFFFFu, updates, o);
-  if (lane == 0 && updates) atomicAdd(&st->seeds, (unsigned long long)updates);
+  if (lane == 0 && updates) add_count(st, kCountSeeds, updates);
+}
+
+template <int SIGN, bool MULTI>
+__global__ void k_seed(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t T,
+                       unsigned long long* keys, uint32_t* status, PropState* st, uint2* chunks) {
+  const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t >= T) return;
+  const GridK& g = grid_of_tri<MULTI>(gs, t);
+  const TriRec r = tris[t];
+  int mn[3], ext[3];
+  seed_box(g, r, mn, ext);
+  if (ext[0] <= 0 || ext[1] <= 0 || ext[2] <= 0) return;
+  const unsigned long long total = (unsigned long long)ext[0] * ext[1] * ext[2];
+  if (split_box(t, total, 0u, 1u, &st->big_seeds, chunks)) return;
+  seed_cells<SIGN>(g, r, t, mn, ext, 0, total, keys, status, st);
+}
+
+template <int SIGN, bool MULTI>
+__global__ void k_seed_chunks(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris,
+                              unsigned long long* keys, uint32_t* status, PropState* st,
+                              const uint2* __restrict__ chunks) {
+  const uint32_t n = min(st->big_seeds, kMaxChunks), warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const uint2 ch = chunks[i];
+    if (ch.x == kNoChunk) continue;
+    const GridK& g = grid_of_tri<MULTI>(gs, ch.x);
+    const TriRec r = tris[ch.x];
+    int mn[3], ext[3];
+    seed_box(g, r, mn, ext);
+    const unsigned long long total = (unsigned long long)ext[0] * ext[1] * ext[2];
+    const unsigned long long k0 = (unsigned long long)ch.y * kChunkCells;
+    seed_cells<SIGN>(g, r, ch.x, mn, ext, k0, min(total, k0 + kChunkCells), keys, status, st);
+  }
 }
 
 // Distance bucket of a state, in its own grid's cell units: u = |d| / (a
@@ -456,15 +562,6 @@ __device__ __forceinline__ uint32_t bucket_of(float inv_delta, float d) {
   const uint32_t b = __float_as_uint(u);   // u > 32: exponent >= 5; +inf has exponent 128
   const uint64_t lin = ((uint64_t)((b >> 23) - 127 - 5) << 23) | (b & 0x7FFFFFu);
   return 32u + (uint32_t)((kLogBuckets * lin) >> 23);
-}
-
-__global__ void k_state_init(PropState* st) {
-  st->b = 0;
-  st->B = 0;
-  for (int k = 0; k < kRing; ++k) st->slot[k] = k;
-  st->cur = kCur0;
-  st->fp = 0;
-  st->far_min[0] = st->far_min[1] = kNoBucket;
 }
 
 // Appends (cell, triangle) of bucket nb: inside the window to its bucket's list
@@ -616,12 +713,6 @@ __global__ void k_collect(const __grid_constant__ GridSet gs, const unsigned lon
 // difference, which stays right when the counter wraps: while a block waits
 // at barrier g, barrier g - 1 is complete and no block is past g + 1, so
 // its difference stays inside (-blocks, blocks).
-constexpr unsigned int kMaxBarrierBlocks = 2048;
-struct GridBarrier {
-  unsigned int arrivals;
-  unsigned int abort;
-  unsigned int pad0[30];
-};
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
   unsigned int v;
@@ -1506,14 +1597,14 @@ __global__ void __launch_bounds__(FILTER ? kSmallBlock : kBigBlock, FILTER ? 3 :
   }
   if (nan) atomicOr(status, bit(M2S_ERR_NAN_DISTANCE));
   for (int o = 16; o; o >>= 1) evals += __shfl_xor_sync(0xFFFFFFFFu, evals, o);
-  if (lane == 0 && evals) atomicAdd(&st->evals, evals);
+  if (lane == 0 && evals) add_count(st, kCountEvals, evals);
   unsigned long long ds = dropped_same, db = dropped_bound;
   for (int o = 16; o; o >>= 1) {
     ds += __shfl_xor_sync(0xFFFFFFFFu, ds, o);
     db += __shfl_xor_sync(0xFFFFFFFFu, db, o);
   }
-  if (lane == 0 && ds) atomicAdd(&st->filter_same, ds);
-  if (lane == 0 && db) atomicAdd(&st->filter_bound, db);
+  if (lane == 0 && ds) add_count(st, kCountSame, ds);
+  if (lane == 0 && db) add_count(st, kCountBound, db);
   if (aborted && lead_block && threadIdx.x == 0) atomicOr(status, bit(M2S_ERR_LIMIT));
   if (lead_block && threadIdx.x == 0) {
     st->round = sh.round;
@@ -1548,37 +1639,44 @@ __device__ __forceinline__ void lattice_range(const GridK& g, int d, float lo, f
   if (fb_ < 0.0f || fa_ > (float)(g.n[d] - 1)) *b = *a - 1;  // no lattice point in range
 }
 
-// With AUDIT, each ray test is also audited (m2s_audit.cuh): the f32
-// decision toggles `bits` exactly as without, the FP64 one toggles `bits64`.
-template <int AXIS, bool MULTI, bool AUDIT = false>
-__global__ void k_rays(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t T, uint32_t* bits,
-                       PropState* st, uint32_t* bits64 = nullptr) {
+// The rectangle of ray origins (low-face cells) that triangle r's padded box
+// covers, along axes IY and IZ; false when it is empty.
+template <int AXIS>
+__device__ __forceinline__ bool ray_box(const GridK& g, const TriRec& r, int* j0, int* k0, uint32_t* nk,
+                                        unsigned long long* total) {
   constexpr int IY = (AXIS + 1) % 3, IZ = (AXIS + 2) % 3;
-  const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (t >= T) return;
-  const GridK& g = grid_of_tri<MULTI>(gs, t);
-  TriRec r = tris[t];
-  P3 a = p3(r.a), b = p3(r.b), c = p3(r.c);
   P3 lo, hi;
-  padded_box(a, b, c, &lo, &hi);
-  int j0, j1, k0, k1;
-  lattice_range(g, IY, vget(lo, IY), vget(hi, IY), &j0, &j1);
-  lattice_range(g, IZ, vget(lo, IZ), vget(hi, IZ), &k0, &k1);
-  if (j1 < j0 || k1 < k0) return;
-  const int nj = j1 - j0 + 1, nk = k1 - k0 + 1;
-  const long long total = (long long)nj * nk;
+  padded_box(p3(r.a), p3(r.b), p3(r.c), &lo, &hi);
+  int j1, k1;
+  lattice_range(g, IY, vget(lo, IY), vget(hi, IY), j0, &j1);
+  lattice_range(g, IZ, vget(lo, IZ), vget(hi, IZ), k0, &k1);
+  if (j1 < *j0 || k1 < *k0) return false;
+  *nk = (uint32_t)(k1 - *k0 + 1);
+  *total = (unsigned long long)(j1 - *j0 + 1) * *nk;
+  return true;
+}
+
+// The rays q0 <= q < q1 of triangle r's rectangle, on one warp.  With AUDIT,
+// each ray test is also audited (m2s_audit.cuh): the f32 decision toggles
+// `bits` exactly as without, the FP64 one toggles `bits64`.
+template <int AXIS, bool AUDIT>
+__device__ __forceinline__ void ray_cells(const GridK& g, const TriRec& r, int j0, int k0, uint32_t nk,
+                                          unsigned long long q0, unsigned long long q1, uint32_t* bits, uint32_t* bits64,
+                                          PropState* st) {
+  constexpr int IY = (AXIS + 1) % 3, IZ = (AXIS + 2) % 3;
+  const int lane = threadIdx.x & 31;
+  const P3 a = p3(r.a), b = p3(r.b), c = p3(r.c);
   uint32_t* bitsA = bits + g.bits_off[AXIS];
   const uint32_t W = g.words[AXIS];
   uint32_t hits = 0, tests = 0, ambiguous = 0, disagree = 0;
-  const bool small = total <= 0x7FFFFFFFll;  // 32-bit division (64-bit costs ~4x the instructions)
-  for (long long q = lane; q < total; q += 32) {
+  const bool small = q1 <= 0x7FFFFFFFull;  // 32-bit division (64-bit costs ~4x the instructions)
+  for (unsigned long long q = q0 + lane; q < q1; q += 32) {
     int c3[3];
     c3[AXIS] = 0;
     if (small) {
-      const uint32_t uq = (uint32_t)q, row = uq / (uint32_t)nk;
+      const uint32_t uq = (uint32_t)q, row = uq / nk;
       c3[IY] = j0 + (int)row;
-      c3[IZ] = k0 + (int)(uq - row * (uint32_t)nk);
+      c3[IZ] = k0 + (int)(uq - row * nk);
     } else {
       c3[IY] = j0 + (int)(q / nk);
       c3[IZ] = k0 + (int)(q % nk);
@@ -1615,7 +1713,7 @@ __global__ void k_rays(const __grid_constant__ GridSet gs, const TriRec* __restr
     atomicXor(&bitsA[col * W + (k >> 5)], 1u << (k & 31));
   }
   for (int o = 16; o; o >>= 1) hits += __shfl_xor_sync(0xFFFFFFFFu, hits, o);
-  if (lane == 0 && hits) atomicAdd(&st->ray_hits, (unsigned long long)hits);
+  if (lane == 0 && hits) add_count(st, kCountRayHits, hits);
   if constexpr (AUDIT) {
     for (int o = 16; o; o >>= 1) {
       tests += __shfl_xor_sync(0xFFFFFFFFu, tests, o);
@@ -1627,6 +1725,55 @@ __global__ void k_rays(const __grid_constant__ GridSet gs, const TriRec* __restr
       atomicAdd(&st->audit[1], (unsigned long long)ambiguous);
       atomicAdd(&st->audit[2], (unsigned long long)disagree);
     }
+  }
+}
+
+// One warp per (triangle, axis = blockIdx.y); large rectangles are split as in k_seed.
+template <int AXIS, bool MULTI, bool AUDIT>
+__device__ __forceinline__ void rays_of(const GridSet& gs, const TriRec* __restrict__ tris, uint32_t t, uint32_t* bits,
+                                        uint32_t* bits64, PropState* st, uint2* chunks) {
+  const GridK& g = grid_of_tri<MULTI>(gs, t);
+  const TriRec r = tris[t];
+  int j0, k0;
+  uint32_t nk;
+  unsigned long long total;
+  if (!ray_box<AXIS>(g, r, &j0, &k0, &nk, &total)) return;
+  if (split_box(t, total, AXIS, 4u, &st->big_rays, chunks)) return;
+  ray_cells<AXIS, AUDIT>(g, r, j0, k0, nk, 0, total, bits, bits64, st);
+}
+template <bool MULTI, bool AUDIT>
+__global__ void k_rays(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t T, uint32_t* bits,
+                       PropState* st, uint32_t* bits64, uint2* chunks) {
+  const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t >= T) return;
+  if (blockIdx.y == 0) rays_of<0, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks);
+  else if (blockIdx.y == 1) rays_of<1, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks);
+  else rays_of<2, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks);
+}
+
+template <int AXIS, bool MULTI, bool AUDIT>
+__device__ __forceinline__ void ray_chunk(const GridSet& gs, const TriRec* __restrict__ tris, uint2 ch, uint32_t* bits,
+                                          uint32_t* bits64, PropState* st) {
+  const GridK& g = grid_of_tri<MULTI>(gs, ch.x);
+  const TriRec r = tris[ch.x];
+  int j0, k0;
+  uint32_t nk;
+  unsigned long long total;
+  if (!ray_box<AXIS>(g, r, &j0, &k0, &nk, &total)) return;
+  const unsigned long long q0 = (unsigned long long)(ch.y >> 2) * kChunkCells;
+  ray_cells<AXIS, AUDIT>(g, r, j0, k0, nk, q0, min(total, q0 + kChunkCells), bits, bits64, st);
+}
+template <bool MULTI, bool AUDIT>
+__global__ void k_ray_chunks(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t* bits,
+                             PropState* st, uint32_t* bits64, const uint2* __restrict__ chunks) {
+  const uint32_t n = min(st->big_rays, kMaxChunks), warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const uint2 ch = chunks[i];
+    if (ch.x == kNoChunk) continue;
+    const uint32_t axis = ch.y & 3u;
+    if (axis == 0u) ray_chunk<0, MULTI, AUDIT>(gs, tris, ch, bits, bits64, st);
+    else if (axis == 1u) ray_chunk<1, MULTI, AUDIT>(gs, tris, ch, bits, bits64, st);
+    else ray_chunk<2, MULTI, AUDIT>(gs, tris, ch, bits, bits64, st);
   }
 }
 
@@ -1681,7 +1828,8 @@ __global__ void k_audit_cells(const __grid_constant__ GridSet gs, const TriRec* 
 // Toggle bits -> suffix parity: bit i becomes the XOR of toggles i..n-1, i.e.
 // the parity of the hits whose cell range 0..=k covers cell i.
 template <bool MULTI>
-__global__ void k_suffix(const __grid_constant__ GridSet gs, int axis, uint32_t* bits) {
+__global__ void k_suffix(const __grid_constant__ GridSet gs, uint32_t* bits) {
+  const int axis = (int)blockIdx.y;
   SegCursor<unsigned long long> sc;
   const unsigned long long ncols = gs.ncols[axis];
   for (unsigned long long col = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; col < ncols;
@@ -1706,7 +1854,17 @@ __global__ void k_suffix(const __grid_constant__ GridSet gs, int axis, uint32_t*
 
 template <int SIGN, bool MULTI>
 __global__ void k_finalize(const __grid_constant__ GridSet gs, const unsigned long long* __restrict__ keys,
-                           const uint32_t* __restrict__ bits, float* __restrict__ out) {
+                           const uint32_t* __restrict__ bits, float* __restrict__ out, PropState* st) {
+  if (blockIdx.x == 0 && threadIdx.x < kParts) {
+    unsigned long long* const sum[kCounts] = {&st->seeds, &st->ray_hits, &st->evals, &st->filter_same,
+                                              &st->filter_bound};
+#pragma unroll
+    for (int c = 0; c < kCounts; ++c) {
+      unsigned long long n = st->parts[c][threadIdx.x].n;
+      for (int o = 16; o; o >>= 1) n += __shfl_xor_sync(0xFFFFFFFFu, n, o);
+      if (threadIdx.x == 0) *sum[c] = n;
+    }
+  }
   SegCursor<uint32_t> sc;
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < gs.ncell;
        i += (unsigned long long)gridDim.x * blockDim.x) {
@@ -1801,6 +1959,7 @@ struct GridJob::Impl {
   DevBuf<float> slack;
   bool filter = false;
   bool audit = false;          // FP64 audit (reports only)
+  DevBuf<uint2> chunks;        // pieces of large triangles (seeding, then rays)
   DevBuf<uint32_t> bits64;     // the audit's FP64-decided ray parities
 };
 
@@ -1826,7 +1985,7 @@ uint32_t GridJob::threads() const { return p->threads; }
 uint64_t GridJob::device_bytes() const {
   const Impl& J = *p;
   return J.comb_tris.n * sizeof(TriRec) + J.tri_grid.n * 4 + J.keys.n * 8 + J.bits.n * 4 +
-         J.bounds.n * sizeof(TriBound) + J.slack.n * 4 +
+         J.chunks.n * sizeof(uint2) + J.bounds.n * sizeof(TriBound) + J.slack.n * 4 +
          (uint64_t)kLists * J.cap * 8 + 2ull * J.cap * 4 + J.table.n * sizeof(GridK);
 }
 
@@ -1847,7 +2006,7 @@ uint32_t default_list_capacity(uint64_t cells) {
 uint64_t grid_job_bytes(uint64_t cells) {
   const uint64_t cap = default_list_capacity(cells);
   const uint64_t ray_words = 3 * (cells / 32 + 3 * std::cbrt((double)cells) * std::cbrt((double)cells));
-  return 8 * cells + (uint64_t)kLists * 8 * cap + 8 * cap + 4 * ray_words + (1u << 20);  // + 68 B per triangle
+  return 8 * cells + (uint64_t)kLists * 8 * cap + 8 * cap + 4 * ray_words + (3u << 20);  // + 68 B per triangle
 }
 
 int check_grid(const GridDesc& g) {
@@ -1955,6 +2114,7 @@ int GridJob::prepare(const MeshView* meshes, uint32_t n, const GridDesc* gds, in
   J.filter = tune.bound_filter;
   J.audit = tune.fp64_audit;
   if (tris && ((st = J.bounds.alloc(tris, s)) || (st = J.slack.alloc(tris, s)))) return st;
+  if (tris && (st = J.chunks.alloc(kMaxChunks, s))) return st;
   if (sign == M2S_SIGN_RAYCAST && (st = J.bits.alloc(woff, s))) return st;
   if (sign == M2S_SIGN_RAYCAST && J.audit && (st = J.bits64.alloc(woff, s))) return st;
   J.cap = tune.list_capacity ? tune.list_capacity : default_list_capacity(N);
@@ -2004,25 +2164,27 @@ int GridJob::enqueue(cudaStream_t s, cudaEvent_t* ev) {
   };
   int st;
   if ((st = mark(0))) return st;
-  M2S_CUDA(cudaMemsetAsync(J.state.p, 0, sizeof(PropState), s));
-  k_state_init<<<1, 1, 0, s>>>(J.state.p);
-  k_fill_u64<<<blocks_for(N, 256), 256, 0, s>>>(J.keys.p, N, KEY_EMPTY);
-  J.launches += 2;
+  k_init<<<blocks_for(N / 2 + 1, 256), 256, 0, s>>>(reinterpret_cast<ulonglong2*>(J.keys.p), N, J.state.p, J.bar.p,
+                                                    J.bits.p, J.bits64.p, raycast ? J.ray_words : 0ull);
+  ++J.launches;
+  const unsigned chunk_blocks = 148u * 8u;
   if (J.T > 0) {
     const unsigned sb = (unsigned)((J.T * 32ull + 255) / 256);
-    if (raycast) {
-      if (multi) k_seed<M2S_SIGN_RAYCAST, true><<<sb, 256, 0, s>>>(J.gs, J.tris, J.T, J.keys.p, J.d_status, J.state.p);
-      else k_seed<M2S_SIGN_RAYCAST, false><<<sb, 256, 0, s>>>(J.gs, J.tris, J.T, J.keys.p, J.d_status, J.state.p);
-    } else {
-      if (multi) k_seed<M2S_SIGN_NORMAL, true><<<sb, 256, 0, s>>>(J.gs, J.tris, J.T, J.keys.p, J.d_status, J.state.p);
-      else k_seed<M2S_SIGN_NORMAL, false><<<sb, 256, 0, s>>>(J.gs, J.tris, J.T, J.keys.p, J.d_status, J.state.p);
-    }
-    ++J.launches;
+    auto seed = [&](auto sign_tag, auto multi_tag) {
+      constexpr int S = decltype(sign_tag)::value;
+      constexpr bool M = decltype(multi_tag)::value;
+      k_seed<S, M><<<sb, 256, 0, s>>>(J.gs, J.tris, J.T, J.keys.p, J.d_status, J.state.p, J.chunks.p);
+      k_seed_chunks<S, M><<<chunk_blocks, 256, 0, s>>>(J.gs, J.tris, J.keys.p, J.d_status, J.state.p, J.chunks.p);
+    };
+    using Ray = std::integral_constant<int, M2S_SIGN_RAYCAST>;
+    using Nor = std::integral_constant<int, M2S_SIGN_NORMAL>;
+    if (raycast) multi ? seed(Ray{}, std::true_type{}) : seed(Ray{}, std::false_type{});
+    else multi ? seed(Nor{}, std::true_type{}) : seed(Nor{}, std::false_type{});
+    J.launches += 2;
   }
   M2S_CUDA(cudaGetLastError());
   if ((st = mark(1))) return st;
   if (J.T > 0) {
-    M2S_CUDA(cudaMemsetAsync(J.bar.p, 0, sizeof(GridBarrier), s));
     if (J.filter) {
       k_bounds<<<blocks_for(J.T, 256), 256, 0, s>>>(J.tris, J.T, J.bounds.p, J.slack.p);
       ++J.launches;
@@ -2055,49 +2217,32 @@ int GridJob::enqueue(cudaStream_t s, cudaEvent_t* ev) {
   if ((st = mark(2))) return st;
   const unsigned fb = blocks_for(N, 256, 148u * 32u);
   if (raycast) {
-    M2S_CUDA(cudaMemsetAsync(J.bits.p, 0, J.ray_words * 4, s));
-    if (J.audit) M2S_CUDA(cudaMemsetAsync(J.bits64.p, 0, J.ray_words * 4, s));
     if (J.T > 0) {
-      const unsigned rb = (unsigned)((J.T * 32ull + 255) / 256);
-      uint32_t* b64 = J.bits64.p;
-      if (J.audit) {
-        if (multi) {
-          k_rays<0, true, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, b64);
-          k_rays<1, true, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, b64);
-          k_rays<2, true, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, b64);
-        } else {
-          k_rays<0, false, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, b64);
-          k_rays<1, false, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, b64);
-          k_rays<2, false, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, b64);
-        }
-      } else if (multi) {
-        k_rays<0, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p);
-        k_rays<1, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p);
-        k_rays<2, true><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p);
-      } else {
-        k_rays<0, false><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p);
-        k_rays<1, false><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p);
-        k_rays<2, false><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p);
-      }
-      J.launches += 3;
+      const dim3 rb((unsigned)((J.T * 32ull + 255) / 256), 3);
+      auto rays = [&](auto multi_tag, auto audit_tag) {
+        constexpr bool M = decltype(multi_tag)::value, A = decltype(audit_tag)::value;
+        k_rays<M, A><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, J.bits64.p, J.chunks.p);
+        k_ray_chunks<M, A><<<chunk_blocks, 256, 0, s>>>(J.gs, J.tris, J.bits.p, J.state.p, J.bits64.p, J.chunks.p);
+      };
+      if (J.audit) multi ? rays(std::true_type{}, std::true_type{}) : rays(std::false_type{}, std::true_type{});
+      else multi ? rays(std::true_type{}, std::false_type{}) : rays(std::false_type{}, std::false_type{});
+      J.launches += 2;
     }
-    for (int a = 0; a < 3; ++a) {
-      if (multi) k_suffix<true><<<blocks_for(J.gs.ncols[a], 256), 256, 0, s>>>(J.gs, a, J.bits.p);
-      else k_suffix<false><<<blocks_for(J.gs.ncols[a], 256), 256, 0, s>>>(J.gs, a, J.bits.p);
-      if (J.audit) {
-        if (multi) k_suffix<true><<<blocks_for(J.gs.ncols[a], 256), 256, 0, s>>>(J.gs, a, J.bits64.p);
-        else k_suffix<false><<<blocks_for(J.gs.ncols[a], 256), 256, 0, s>>>(J.gs, a, J.bits64.p);
-      }
+    const dim3 xb(blocks_for(std::max(J.gs.ncols[0], std::max(J.gs.ncols[1], J.gs.ncols[2])), 256), 3);
+    for (uint32_t* words : {J.bits.p, J.audit ? J.bits64.p : nullptr}) {
+      if (!words) continue;
+      if (multi) k_suffix<true><<<xb, 256, 0, s>>>(J.gs, words);
+      else k_suffix<false><<<xb, 256, 0, s>>>(J.gs, words);
+      ++J.launches;
     }
-    J.launches += J.audit ? 6 : 3;
     M2S_CUDA(cudaGetLastError());
     if ((st = mark(3))) return st;
-    if (multi) k_finalize<M2S_SIGN_RAYCAST, true><<<fb, 256, 0, s>>>(J.gs, J.keys.p, J.bits.p, J.d_out);
-    else k_finalize<M2S_SIGN_RAYCAST, false><<<fb, 256, 0, s>>>(J.gs, J.keys.p, J.bits.p, J.d_out);
+    if (multi) k_finalize<M2S_SIGN_RAYCAST, true><<<fb, 256, 0, s>>>(J.gs, J.keys.p, J.bits.p, J.d_out, J.state.p);
+    else k_finalize<M2S_SIGN_RAYCAST, false><<<fb, 256, 0, s>>>(J.gs, J.keys.p, J.bits.p, J.d_out, J.state.p);
   } else {
     if ((st = mark(3))) return st;
-    if (multi) k_finalize<M2S_SIGN_NORMAL, true><<<fb, 256, 0, s>>>(J.gs, J.keys.p, nullptr, J.d_out);
-    else k_finalize<M2S_SIGN_NORMAL, false><<<fb, 256, 0, s>>>(J.gs, J.keys.p, nullptr, J.d_out);
+    if (multi) k_finalize<M2S_SIGN_NORMAL, true><<<fb, 256, 0, s>>>(J.gs, J.keys.p, nullptr, J.d_out, J.state.p);
+    else k_finalize<M2S_SIGN_NORMAL, false><<<fb, 256, 0, s>>>(J.gs, J.keys.p, nullptr, J.d_out, J.state.p);
   }
   M2S_CUDA(cudaGetLastError());
   ++J.launches;
@@ -2119,7 +2264,7 @@ int GridJob::read_state(cudaStream_t s, GridRunInfo* info) {
   Impl& J = *p;
   PropState* h = host_state();
   if (!h) return M2S_ERR_OUT_OF_MEMORY;
-  M2S_CUDA(cudaMemcpyAsync(h, J.state.p, sizeof(PropState), cudaMemcpyDeviceToHost, s));
+  M2S_CUDA(cudaMemcpyAsync(h, J.state.p, offsetof(PropState, parts), cudaMemcpyDeviceToHost, s));
   M2S_CUDA(cudaStreamSynchronize(s));
   info->overflow = (h->overflow | h->overflow2[0] | h->overflow2[1]) != 0;
   info->seeds = h->seeds;
