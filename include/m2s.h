@@ -360,19 +360,14 @@ int m2s_last_grid_phase_ms(float out[4]);
  * copying up to `capacity` steps (2 * capacity words) to `out` (may be NULL). */
 uint32_t m2s_last_grid_round_log(uint32_t* out, uint32_t capacity);
 
-/* Point queries run one thread per query (from 2^19 queries the 32 queries of
- * a warp walk the tree together, the budget still counted per query); a
+/* Point queries run one thread per query (from 2^17 queries the 32 queries of
+ * a warp start down the tree together, the budget still counted per query); a
  * query that visits more than its node budget is continued by a whole warp
- * (points deep inside a closed mesh
- * see most triangles at nearly the same distance).  `node_visits` is the
- * budget of batches of 2^20 queries and more; a batch of nq queries from 2^18
- * uses node_visits * sqrt(nq / 2^20), and a smaller one node_visits / 16,
- * at least 64 either way, since a small batch's time is its longest
- * single-thread search.  0 keeps every query on one thread.
- * Bvh(Normal) hands searches and band folds over the budget to the warp pass
- * in batches under 2^18 queries, and at every size when node_visits is 64 or
- * less (a win on closed meshes with many deep-interior points, a loss on open
- * surfaces; the autotuner tries it).
+ * (Bvh(Normal): its tie-band fold too).  `node_visits` is the budget of
+ * batches of 2^20 queries and more; a batch of nq queries from 2^18 uses
+ * node_visits * sqrt(nq / 2^20) and a smaller one node_visits * nq / 2^19, at
+ * least 24, since a small batch's time is its longest single-thread search.  0
+ * keeps every query on one thread.
  * Process-wide tuning knob; the autotuner sets it. */
 void m2s_set_query_budget(uint32_t node_visits);
 uint32_t m2s_query_budget(void);

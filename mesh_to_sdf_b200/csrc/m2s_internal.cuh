@@ -31,17 +31,51 @@ struct __align__(16) TriRec {
 // Internal LBVH node, 64 bytes: both child boxes live in the parent so one
 // node fetch tests both children.  l_lo.w / l_hi.w hold the left / right
 // child references (uint bits); LEAF_BIT marks a leaf (index into the
-// LBVH-ordered triangle array).
+// LBVH-ordered triangle array).  r_lo.w / r_hi.w hold the squared distances up
+// to which the left / right child's pillbox may prune (0: never).
 struct __align__(16) BvhNode {
   float4 l_lo, l_hi, r_lo, r_hi;
 };
 constexpr uint32_t LEAF_BIT = 0x80000000u;
+
+// A second bound of a node's children, 32 bytes each (left, then right): a
+// pillbox that holds the child's triangles, centre c, unit axis n, half height
+// h and radius r.  An axis-aligned box is loose by about a triangle's size, so
+// for a point far from the mesh every leaf within that much of the nearest
+// distance is visited; a patch of a surface is flat, and its pillbox is loose
+// by the patch's sagitta only.  Searches prune by both bounds (pill_dist2 in
+// m2s_query.cu).
+//   a : c.xyz | h and r rounded up to 16 bits each (h high), slack included
+//   b : n.xyz | squared distance up to which the bound may prune (0: never; also in the node)
+struct __align__(16) Pill {
+  float4 a, b;
+};
+// Children of more leaves than this have no pillbox (a large patch is not
+// flat, and building it would read every leaf once per level).
+constexpr uint32_t kPillLeaves = 256;
+// A pillbox prunes a search whose best distance is at most this many times
+// the smallest Q of its triangles, Q = (twice the area) * (shortest edge) /
+// (longest edge)^2.  The reference's f32 closest point (closest_point_proper)
+// can leave a triangle only in the face region, when rounding hides that the
+// foot of the perpendicular lies outside an edge line: by at most
+// o = 24 u D^2 / Q at distance D (u = 2^-24: each of the products d1 d4 - d3 d2
+// errs by 24 u (longest edge)^2 D^2), which brings the point nearer than the
+// triangle by o^2 / (2 D).  At D = 1024 Q that is below 20 u D, well inside
+// the slack of 2^-17 = 128 u of the coordinates' magnitudes.  In every other
+// region the point lies on the triangle up to rounding.
+constexpr float kPillReach = 1024.0f;
+// Slack of a pillbox per unit of coordinate magnitude: the node's share is in
+// h and r, the query's is added by the search.
+constexpr float kPillSlack = 0x1p-17f;
+// A pillbox is used when its half height is below this share of the box's.
+constexpr float kPillFlat = 0.5f;
 
 // Device view of a resident mesh.
 struct MeshView {
   const TriRec* tris;    // crate triangle order
   const TriRec* stris;   // LBVH leaf order
   const BvhNode* nodes;  // n_tris - 1 internal nodes (node 0 is the root)
+  const Pill* pills;     // two per internal node
   uint32_t n_tris;
   uint32_t root;  // 0, or LEAF_BIT | 0 for a single triangle
 };
@@ -104,9 +138,10 @@ struct MeshInput {
 struct DeviceMesh {
   DevBuf<TriRec> tris, stris;
   DevBuf<BvhNode> nodes;
+  DevBuf<Pill> pills;
   uint32_t n_tris = 0;
   uint32_t root = 0;
-  MeshView view() const { return {tris.p, stris.p, nodes.p, n_tris, root}; }
+  MeshView view() const { return {tris.p, stris.p, nodes.p, pills.p, n_tris, root}; }
 };
 
 // Builds the triangle records and the LBVH.  d_status receives status bits.
@@ -131,29 +166,24 @@ int query_points(const MeshView& m, int accel, int sign, const float* d_q, uint6
 // continued one warp per query (0 disables the second pass).
 extern std::atomic<uint32_t> g_query_budget;
 // The budget a batch of nq queries uses: `base` from 2^20 queries up,
-// base * sqrt(nq / 2^20) from 2^18, and base / 16 below, at least 64 (0 stays
-// 0: no warp pass).  Below 2^18 queries every query has a thread from the
-// start and the batch waits for its longest searches, which the warp pass
-// finishes sooner (star s6 mixed points, Rtree, base 1024: 50,000 queries
-// 1.30 -> 1.08 ms, 100,000 1.68 -> 1.51 ms); from 2^18 on, the thread pass's
-// throughput counts (400,000: 3.32 ms at 632 against 3.83 at 316 and 3.99 at 158).
+// base * sqrt(nq / 2^20) from 2^18 and base * nq / 2^19 below, at least 24 (0
+// stays 0: no warp pass).  A batch whose queries all have a thread from the
+// start waits for its longest searches, which the warp pass finishes sooner;
+// the more queries, the more the thread pass's throughput counts (budgets 24 /
+// 64 / 128 / 192: star s6, RtreeBvh, 20,000 queries 0.35 / 0.39 / 0.43 / 0.45
+// ms, 100,000 0.88 / 0.75 / 0.58 / 0.61; the terrain strip, Rtree, 20,000
+// 0.31 / 0.39 / 0.50 / 0.61 ms, 130,000 1.41 / 1.37 / 1.28 / 1.23; star s6,
+// Bvh(Normal), 100,000 1.50 / 1.15 / 0.67 / 0.71).
 inline uint32_t effective_query_budget(uint32_t base, uint64_t nq) {
   if (base == 0) return 0;
-  const double f = nq >= (1ull << 20) ? 1.0
+  const double f = nq >= (1ull << 20)   ? 1.0
                    : nq >= (1ull << 18) ? std::sqrt((double)nq / (double)(1ull << 20))
-                                        : 1.0 / 16.0;
-  const uint32_t b = (uint32_t)(base * f + 0.5);
-  return b < 64 ? std::min<uint32_t>(64, base) : b;
+                                        : (double)nq / (double)(1ull << 19);
+  return std::max((uint32_t)(base * f + 0.5), std::min<uint32_t>(24, base));
 }
-// Node budgets the query autotuner tries (64 also moves Bvh(Normal) batches
-// of 2^18 queries and more to the warp hand-off: see query_points).
+// Node budgets the query autotuner tries.
 constexpr int kQueryBudgetCandidates = 8;
 constexpr uint32_t kQueryBudgets[kQueryBudgetCandidates] = {0, 64, 256, 512, 1024, 1536, 2048, 4096};
-// Base budgets at or below this hand Bvh(Normal) searches and band folds to
-// the warp pass at every batch size; larger ones keep batches of 2^18
-// queries and more in one pass.
-constexpr uint32_t kNormalHandoffMaxBudget = 64;
-
 // Profiling (m2s_set_profiling, per host thread): whether it is on, and the
 // traversal counts of the last point query made with it on:
 // [queries, search node fetches, search triangle tests, sign node fetches,

@@ -273,7 +273,7 @@ __device__ __forceinline__ int kdelta(const uint32_t* __restrict__ k, int n, int
 }
 
 __global__ void k_karras(const uint32_t* __restrict__ keys, int n, BvhNode* nodes, uint32_t* node_parent,
-                         uint32_t* leaf_parent) {
+                         uint32_t* leaf_parent, uint2* range) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
   int d = (kdelta(keys, n, i, i + 1) - kdelta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -291,6 +291,7 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, int n, BvhNode* node
     if (kdelta(keys, n, i, (int)(i + (s + t) * d)) > dnode) s += t;
   } while (t > 1);
   int gamma = (int)(i + s * d + min(d, 0));
+  range[i] = make_uint2((uint32_t)min(i, j), (uint32_t)max(i, j));  // the node's leaves
   uint32_t left = (min(i, j) == gamma) ? (LEAF_BIT | (uint32_t)gamma) : (uint32_t)gamma;
   uint32_t right = (max(i, j) == gamma + 1) ? (LEAF_BIT | (uint32_t)(gamma + 1)) : (uint32_t)(gamma + 1);
   nodes[i].l_lo.w = __uint_as_float(left);
@@ -343,6 +344,149 @@ __global__ void k_refit(const float4* __restrict__ boxes, const uint32_t* __rest
     if (up == 0xFFFFFFFFu) return;
     child = p;
     p = up;
+  }
+}
+
+// ---- pillboxes ---------------------------------------------------------------
+// Leaves first .. last of the tree under one pillbox, by `lanes` lanes of a
+// warp (1 or 32; lane k takes leaves first + k, first + k + lanes, ...).  The
+// axis is the sum of the triangles' area vectors, turned to the side of the
+// first (a strip's windows alternate); the extents are those of the vertices
+// about the stored centre and axis.
+template <int LANES>
+__device__ __forceinline__ Pill make_pill(const TriRec* __restrict__ stris, uint32_t first, uint32_t last, uint32_t lane) {
+  auto sum = [&](float v) {
+    if (LANES > 1)
+      for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    return v;
+  };
+  auto most = [&](float v) {
+    if (LANES > 1)
+      for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+    return v;
+  };
+  auto area = [](const TriRec& t) {
+    const float ux = t.b.x - t.a.x, uy = t.b.y - t.a.y, uz = t.b.z - t.a.z;
+    const float vx = t.c.x - t.a.x, vy = t.c.y - t.a.y, vz = t.c.z - t.a.z;
+    return P3{uy * vz - uz * vy, uz * vx - ux * vz, ux * vy - uy * vx};
+  };
+  const P3 ref = area(stris[first]);
+  float nx = 0.f, ny = 0.f, nz = 0.f, limit = INFINITY;
+  float lox = INFINITY, loy = INFINITY, loz = INFINITY, hix = -INFINITY, hiy = -INFINITY, hiz = -INFINITY;
+  for (uint32_t k = first + lane; k <= last; k += LANES) {
+    const TriRec t = stris[k];
+    const P3 w = area(t);
+    const float s = w.x * ref.x + w.y * ref.y + w.z * ref.z < 0.f ? -1.f : 1.f;
+    nx += s * w.x;
+    ny += s * w.y;
+    nz += s * w.z;
+    lox = fminf(lox, fminf(t.a.x, fminf(t.b.x, t.c.x)));
+    loy = fminf(loy, fminf(t.a.y, fminf(t.b.y, t.c.y)));
+    loz = fminf(loz, fminf(t.a.z, fminf(t.b.z, t.c.z)));
+    hix = fmaxf(hix, fmaxf(t.a.x, fmaxf(t.b.x, t.c.x)));
+    hiy = fmaxf(hiy, fmaxf(t.a.y, fmaxf(t.b.y, t.c.y)));
+    hiz = fmaxf(hiz, fmaxf(t.a.z, fmaxf(t.b.z, t.c.z)));
+    if (__float_as_int(t.a.w) == TRI_PROPER) {
+      auto len2 = [](float4 p, float4 q) {
+        const float x = p.x - q.x, y = p.y - q.y, z = p.z - q.z;
+        return x * x + y * y + z * z;
+      };
+      const float e0 = len2(t.a, t.b), e1 = len2(t.b, t.c), e2 = len2(t.c, t.a);
+      const float q = sqrtf(w.x * w.x + w.y * w.y + w.z * w.z) * sqrtf(fminf(e0, fminf(e1, e2))) /
+                      fmaxf(e0, fmaxf(e1, e2));
+      limit = q > 0.f ? fminf(limit, q) : 0.f;  // also 0 where the area underflows or anything is NaN
+      if (!(q > 0.f)) limit = 0.f;
+    }
+  }
+  nx = sum(nx);
+  ny = sum(ny);
+  nz = sum(nz);
+  limit = -most(-limit);
+  lox = -most(-lox);
+  loy = -most(-loy);
+  loz = -most(-loz);
+  hix = most(hix);
+  hiy = most(hiy);
+  hiz = most(hiz);
+  const float nn = nx * nx + ny * ny + nz * nz;
+  if (nn > 0.f && nn < INFINITY) {
+    const float inv = 1.0f / sqrtf(nn);
+    nx *= inv;
+    ny *= inv;
+    nz *= inv;
+  }
+  const float one = nx * nx + ny * ny + nz * nz;
+  if (!(one > 0.99999f && one < 1.00001f)) nx = 0.f, ny = 0.f, nz = 1.f;  // no area: any axis is right
+  float cx = 0.5f * (lox + hix), cy = 0.5f * (loy + hiy), cz = 0.5f * (loz + hiz);
+  float omin = INFINITY, omax = -INFINITY;
+  auto along = [&](float4 v) { return (v.x - cx) * nx + (v.y - cy) * ny + (v.z - cz) * nz; };
+  for (uint32_t k = first + lane; k <= last; k += LANES) {
+    const TriRec t = stris[k];
+    const float a = along(t.a), b = along(t.b), c = along(t.c);
+    omin = fminf(omin, fminf(a, fminf(b, c)));
+    omax = fmaxf(omax, fmaxf(a, fmaxf(b, c)));
+  }
+  omin = -most(-omin);
+  omax = most(omax);
+  const float mid = 0.5f * (omin + omax);
+  cx += mid * nx;
+  cy += mid * ny;
+  cz += mid * nz;
+  float h = 0.f, r2 = 0.f;
+  for (uint32_t k = first + lane; k <= last; k += LANES) {
+    const TriRec t = stris[k];
+    for (const float4& v : {t.a, t.b, t.c}) {
+      const float o = along(v), x = v.x - cx, y = v.y - cy, z = v.z - cz, qq = x * x + y * y + z * z;
+      h = fmaxf(h, fabsf(o));
+      r2 = fmaxf(r2, qq * (1.0f + 0x1p-20f) - o * o);
+    }
+  }
+  h = most(h);
+  r2 = most(r2);
+  const float scale = fmaxf(fmaxf(fmaxf(fabsf(lox), fabsf(hix)), fmaxf(fabsf(loy), fabsf(hiy))),
+                            fmaxf(fabsf(loz), fabsf(hiz)));
+  const float slack = kPillSlack * scale;
+  auto up16 = [](float v) { return (__float_as_uint(v) + 0xFFFFu) >> 16; };  // v >= 0
+  const float hs = h + slack, rs = sqrtf(r2) * 1.00001f + slack;
+  const float reach = kPillReach * limit;
+  // NaN or infinite vertices, and magnitudes whose squares overflow: never prune.
+  const bool fine = hs < 0x1p60f && rs < 0x1p60f && scale < 0x1p60f;
+  // Where the pillbox is not much flatter than the box is along its axis, the
+  // box alone prunes about as well: a search then skips it (limit 0).
+  const float flat = 0.5f * ((hix - lox) * fabsf(nx) + (hiy - loy) * fabsf(ny) + (hiz - loz) * fabsf(nz));
+  Pill p;
+  p.a = make_float4(cx, cy, cz, __uint_as_float(fine ? (up16(hs) << 16) | up16(rs) : 0u));
+  p.b = make_float4(nx, ny, nz, fine && h < kPillFlat * flat ? fminf(reach * reach, 0x1p126f) : 0.0f);
+  return p;
+}
+
+constexpr uint32_t kPillThread = 8;  // children of at most this many leaves take one lane, others a warp
+__global__ void k_pills(const TriRec* __restrict__ stris, BvhNode* __restrict__ nodes,
+                        const uint2* __restrict__ range, uint32_t children, Pill* __restrict__ pills) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+  uint32_t first = 0, last = 0;
+  bool wide = false;
+  auto store = [&](const Pill& p) {
+    pills[i] = p;
+    (i & 1u ? nodes[i >> 1].r_hi : nodes[i >> 1].r_lo).w = p.b.w;
+  };
+  if (i < children) {
+    const BvhNode& nd = nodes[i >> 1];
+    const uint32_t gamma = __float_as_uint(nd.l_lo.w) & ~LEAF_BIT;  // the left child's last leaf
+    const uint2 rg = range[i >> 1];
+    first = i & 1u ? gamma + 1u : rg.x;
+    last = i & 1u ? rg.y : gamma;
+    const uint32_t m = last - first + 1u;
+    if (m <= kPillThread) store(make_pill<1>(stris, first, last, 0u));
+    else if (m <= kPillLeaves) wide = true;
+    else store(Pill{make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 1.f, 0.f)});
+  }
+  uint32_t todo = __ballot_sync(0xFFFFFFFFu, wide);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1u;
+    const Pill p = make_pill<32>(stris, __shfl_sync(0xFFFFFFFFu, first, src), __shfl_sync(0xFFFFFFFFu, last, src), lane);
+    if (lane == (uint32_t)src) store(p);
   }
 }
 
@@ -431,14 +575,17 @@ int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, 
   M2S_CUDA(cudaGetLastError());
   if (T < 2) return M2S_OK;
   DevBuf<uint32_t> node_parent, leaf_parent, counters;
-  if ((st = out->nodes.alloc(T - 1, s)) || (st = node_parent.alloc(T - 1, s)) || (st = leaf_parent.alloc(T, s)) ||
+  DevBuf<uint2> range;
+  if ((st = out->nodes.alloc(T - 1, s)) || (st = out->pills.alloc(2ull * (T - 1), s)) || (st = range.alloc(T - 1, s)) || (st = node_parent.alloc(T - 1, s)) || (st = leaf_parent.alloc(T, s)) ||
       (st = counters.alloc(T - 1, s)))
     return st;
   M2S_CUDA(cudaMemsetAsync(counters.p, 0, (T - 1) * sizeof(uint32_t), s));
-  k_karras<<<grid_for(T - 1), kThreads, 0, s>>>(keys.p, (int)T, out->nodes.p, node_parent.p, leaf_parent.p);
+  k_karras<<<grid_for(T - 1), kThreads, 0, s>>>(keys.p, (int)T, out->nodes.p, node_parent.p, leaf_parent.p,
+                                          range.p);
   M2S_CUDA(cudaGetLastError());
   k_refit<<<grid_for(T), kThreads, 0, s>>>(boxes.p, perm.p, (int)T, out->nodes.p, node_parent.p, leaf_parent.p,
                                            counters.p);
+  k_pills<<<grid_for(2ull * (T - 1), 128), 128, 0, s>>>(out->stris.p, out->nodes.p, range.p, 2u * (T - 1), out->pills.p);
   M2S_CUDA(cudaGetLastError());
   return M2S_OK;
 }

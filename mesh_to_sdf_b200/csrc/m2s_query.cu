@@ -256,6 +256,7 @@ __global__ void __launch_bounds__(kBwThreads) k_brute_normal_warp(const TriRec* 
 // ---------------------------------------------------------------------------
 // LBVH traversals.
 constexpr int kStack = 64;
+constexpr uint32_t kNoNode = 0xFFFFFFFFu;
 
 __device__ __forceinline__ float box_dist2(P3 p, float4 lo, float4 hi) {
   float dx = fmaxf(fmaxf(lo.x - p.x, p.x - hi.x), 0.0f);
@@ -279,6 +280,42 @@ __device__ __forceinline__ TriRec load_tri(const TriRec* t, uint32_t i) {
   return {__ldg(f), __ldg(f + 1), __ldg(f + 2)};
 }
 
+// The pillbox bound (Pill, m2s_internal.cuh): a squared distance that no
+// triangle of the child is nearer than, for a query whose slack is ps.  On the
+// star s6's 1M mixed points it takes a search from 292 node fetches and 131
+// triangle tests to 73 and 11 (most of them were leaves at nearly the nearest
+// distance, the longest searches 6,000 nodes), and the batch from 5.8 to 2.4
+// ms; about 25 instructions a child against 110 of a triangle test.  The
+// factor 1 - 2^-20 keeps the lateral distance below the true one whatever the
+// cancellation in |q|^2 - a^2 loses (12 units of roundoff of |q|^2).
+__device__ __forceinline__ Pill load_pill(const Pill* pills, uint32_t i) {
+  const float4* f = reinterpret_cast<const float4*>(pills + i);
+  return {__ldg(f), __ldg(f + 1)};
+}
+__device__ __forceinline__ float pill_query_slack(P3 p) {
+  return kPillSlack * fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z)));
+}
+__device__ __forceinline__ float pill_dist2(const Pill& pl, P3 p, float ps) {
+  const float x = p.x - pl.a.x, y = p.y - pl.a.y, z = p.z - pl.a.z;
+  const float a = fmaf(x, pl.b.x, fmaf(y, pl.b.y, z * pl.b.z));
+  const float qq = fmaf(x, x, fmaf(y, y, z * z));
+  const float l2 = fmaxf(fmaf(-a, a, qq * (1.0f - 0x1p-20f)), 0.0f);
+  float l;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(l) : "f"(l2));
+  const uint32_t w = __float_as_uint(pl.a.w);
+  const float da = fmaxf(fabsf(a) - (__uint_as_float(w & 0xFFFF0000u) + ps), 0.0f);
+  const float dl = fmaxf(l - (__uint_as_float(w << 16) + ps), 0.0f);
+  return fmaf(da, da, dl * dl);
+}
+// Raises d2, the box distance of child i, to its pillbox distance where that
+// may prune a search whose best squared distance is `best` (limit: the node's
+// copy of the pillbox's).
+__device__ __forceinline__ void pill_raise(const Pill* pills, uint32_t i, float limit, P3 p, float ps, float best,
+                                           float* d2) {
+  if (*d2 <= best && best < limit)
+    *d2 = fmaxf(*d2, pill_dist2(load_pill(pills, i), p, ps));  // a NaN bound leaves d2 as it is
+}
+
 struct Nearest {
   float d2;
   uint32_t tri;   // crate triangle index
@@ -298,54 +335,44 @@ struct QCount {
 };
 constexpr int kQueryCounters = 11;
 
-// Exact nearest triangle under the f32 point_triangle_distance2 (geo.rs:33-37),
-// ties to the lowest triangle index.  Boxes are padded by 1e-4 (geo.rs:4-22),
-// which keeps the f32 box test conservative.  Starts from `best` (an upper
-// bound from an earlier, unfinished search, or +inf).  With a budget, the
-// search gives up after `budget` node visits and clears *finished; `best` is
-// then still a valid upper bound for a second pass.
-template <bool STATS = false>
-__device__ Nearest nearest_triangle(const MeshView& m, P3 p, bool* overflow, Nearest best = {INFINITY, 0xFFFFFFFFu, 0},
-                                    uint32_t budget = 0xFFFFFFFFu, bool* finished = nullptr, QCount* qc = nullptr) {
-  auto eval = [&](uint32_t leaf) {
-    if constexpr (STATS) ++qc->tests;
-    TriRec r = load_tri(m.stris, leaf);
-    float d2 = point_triangle_distance2(p, p3(r.a), p3(r.b), p3(r.c), __float_as_int(r.a.w));
-    uint32_t idx = __float_as_uint(r.b.w);
-    if (d2 < best.d2 || (d2 == best.d2 && idx < best.tri)) best = {d2, idx, leaf};
-  };
-  if (finished) *finished = true;
-  if (m.root & LEAF_BIT) {
-    eval(m.root & ~LEAF_BIT);
-    return best;
+// Tests triangle `leaf` (of the LBVH order) against the best so far: exact
+// f32 point_triangle_distance2 (geo.rs:33-37), ties to the lowest triangle index.
+template <bool STATS>
+__device__ __forceinline__ void test_leaf(const MeshView& m, P3 p, uint32_t leaf, Nearest* best, QCount* qc) {
+  if constexpr (STATS) ++qc->tests;
+  TriRec r = load_tri(m.stris, leaf);
+  float d2 = point_triangle_distance2(p, p3(r.a), p3(r.b), p3(r.c), __float_as_int(r.a.w));
+  uint32_t idx = __float_as_uint(r.b.w);
+  if (d2 < best->d2 || (d2 == best->d2 && idx < best->tri)) *best = {d2, idx, leaf};
+}
+
+// One lane's search from `node` (kNoNode: from the top of the stack) down and
+// through its stack of (node, box distance).  Gives up after `budget` node
+// visits in all and returns false; `best` is then still a valid upper bound.
+// The loop has one path through its body and one way back to its top: with
+// `continue`s the lanes of a warp that took different branches never met
+// again and walked the tree one group after another.
+template <bool STATS>
+__device__ __forceinline__ bool walk_lane(const MeshView& m, P3 p, float ps, Nearest* best, uint32_t node,
+                                          uint32_t* st_node, float* st_dist, int sp, uint32_t visits, uint32_t budget,
+                                          bool* overflow, QCount* qc) {
+  while (node == kNoNode && sp > 0) {
+    --sp;
+    if (st_dist[sp] <= best->d2) node = st_node[sp];
   }
-  uint32_t st_node[kStack];
-  float st_dist[kStack];
-  int sp = 0;
-  uint32_t node = 0;
-  uint32_t visits = 0;
-  while (true) {
-    if (++visits > budget) {
-      *finished = false;
-      break;
-    }
+  while (node != kNoNode && visits < budget) {
+    ++visits;
     if constexpr (STATS) ++qc->visits;
     BvhNode nd = load_node(m.nodes, node);
     float dl = box_dist2(p, nd.l_lo, nd.l_hi), dr = box_dist2(p, nd.r_lo, nd.r_hi);
     uint32_t L = __float_as_uint(nd.l_lo.w), R = __float_as_uint(nd.l_hi.w);
-    bool goL = dl <= best.d2, goR = dr <= best.d2;
-    if (goL && (L & LEAF_BIT)) {
-      eval(L & ~LEAF_BIT);
-      goL = false;
-    }
-    if (goR && (R & LEAF_BIT)) {
-      eval(R & ~LEAF_BIT);
-      goR = false;
-    }
-    goL = goL && dl <= best.d2;
-    goR = goR && dr <= best.d2;
+    pill_raise(m.pills, 2u * node, nd.r_lo.w, p, ps, best->d2, &dl);
+    pill_raise(m.pills, 2u * node + 1u, nd.r_hi.w, p, ps, best->d2, &dr);
+    if ((L & LEAF_BIT) && dl <= best->d2) test_leaf<STATS>(m, p, L & ~LEAF_BIT, best, qc);
+    if ((R & LEAF_BIT) && dr <= best->d2) test_leaf<STATS>(m, p, R & ~LEAF_BIT, best, qc);
+    const bool goL = !(L & LEAF_BIT) && dl <= best->d2, goR = !(R & LEAF_BIT) && dr <= best->d2;
+    const bool lfirst = goL && (!goR || dl <= dr);
     if (goL && goR) {
-      bool lfirst = dl <= dr;
       if (sp < kStack) {
         st_node[sp] = lfirst ? R : L;
         st_dist[sp] = lfirst ? dr : dl;
@@ -353,28 +380,32 @@ __device__ Nearest nearest_triangle(const MeshView& m, P3 p, bool* overflow, Nea
       } else {
         *overflow = true;
       }
-      node = lfirst ? L : R;
-      continue;
     }
-    if (goL) {
-      node = L;
-      continue;
-    }
-    if (goR) {
-      node = R;
-      continue;
-    }
-    bool found = false;
-    while (sp > 0) {
+    node = lfirst ? L : (goR ? R : kNoNode);
+    while (node == kNoNode && sp > 0) {
       --sp;
-      if (st_dist[sp] <= best.d2) {
-        node = st_node[sp];
-        found = true;
-        break;
-      }
+      if (st_dist[sp] <= best->d2) node = st_node[sp];
     }
-    if (!found) break;
   }
+  return node == kNoNode;
+}
+
+// Exact nearest triangle.  Boxes are padded by 1e-4 (geo.rs:4-22), which keeps
+// the f32 box test conservative.  Starts from `best` (an upper bound from an
+// earlier, unfinished search, or +inf).  With a budget, the search gives up
+// after `budget` node visits and clears *finished.
+template <bool STATS = false>
+__device__ Nearest nearest_triangle(const MeshView& m, P3 p, bool* overflow, Nearest best = {INFINITY, 0xFFFFFFFFu, 0},
+                                    uint32_t budget = 0xFFFFFFFFu, bool* finished = nullptr, QCount* qc = nullptr) {
+  bool done = true;
+  if (m.root & LEAF_BIT) {
+    test_leaf<STATS>(m, p, m.root & ~LEAF_BIT, &best, qc);
+  } else {
+    uint32_t st_node[kStack];
+    float st_dist[kStack];
+    done = walk_lane<STATS>(m, p, pill_query_slack(p), &best, 0u, st_node, st_dist, 0, 0u, budget, overflow, qc);
+  }
+  if (finished) *finished = done;
   return best;
 }
 
@@ -386,30 +417,41 @@ __device__ Nearest nearest_triangle(const MeshView& m, P3 p, bool* overflow, Nea
 // single-thread search gives (exhaustive under its own bound, ties to the
 // lowest triangle index); `budget` counts the nodes a lane took, and a lane
 // over it stops taking nodes and clears *finished.
+//
+// The warp stays together while a node is taken by kPacketLanes lanes on
+// average (looked at every kPacketCheck nodes); once fewer want it, each lane
+// goes on alone from its own part of the stack.  Queries that lie close
+// together against their distance from the mesh stay together to the end.
+// Measured (never apart / parted below 8, 12, 16 lanes / always apart): 1M
+// RtreeBvh points on star s6 3.2 / 2.9, 2.4, 2.5 / 2.3 ms; 4M Rtree points on
+// the terrain strip 11.2 / 11.4, 11.8, 12.7 / 14.8 ms, 1M 4.3 / 4.0, 3.9, 4.1 / 4.5.
+constexpr uint32_t kPacketCheck = 16, kPacketLanes = 12;
 template <bool STATS = false>
 __device__ Nearest nearest_triangle_packet(const MeshView& m, P3 p, bool active, bool* overflow, uint32_t budget,
                                            bool* finished, QCount* qc = nullptr) {
   Nearest best{INFINITY, 0xFFFFFFFFu, 0};
-  auto eval = [&](uint32_t leaf) {
-    if constexpr (STATS) ++qc->tests;
-    TriRec r = load_tri(m.stris, leaf);
-    float d2 = point_triangle_distance2(p, p3(r.a), p3(r.b), p3(r.c), __float_as_int(r.a.w));
-    uint32_t idx = __float_as_uint(r.b.w);
-    if (d2 < best.d2 || (d2 == best.d2 && idx < best.tri)) best = {d2, idx, leaf};
-  };
+  auto eval = [&](uint32_t leaf) { test_leaf<STATS>(m, p, leaf, &best, qc); };
   *finished = true;
   bool live = active;  // still taking nodes
   if (m.root & LEAF_BIT) {
     if (live) eval(m.root & ~LEAF_BIT);
     return best;
   }
+  const float ps = pill_query_slack(p);
   uint32_t st_node[kStack];
   float st_dist[kStack];
   int sp = 0;
   uint32_t node = 0;
   uint32_t visits = 0;
   bool take = live;  // this lane wants `node`
+  uint32_t walked = 0, taken = 0;  // nodes the warp walked, lanes that took them
   while (true) {
+    if (++walked % kPacketCheck == 0u && taken < kPacketLanes * walked) {
+      const bool more = walk_lane<STATS>(m, p, ps, &best, take && live ? node : kNoNode, st_node, st_dist,
+                                         live ? sp : 0, visits, budget, overflow, qc);
+      if (!more) *finished = false;
+      break;
+    }
     if (take) {
       if (++visits > budget) {
         *finished = false;
@@ -419,17 +461,27 @@ __device__ Nearest nearest_triangle_packet(const MeshView& m, P3 p, bool active,
       }
     }
     take = take && live;
-    if (__any_sync(0xFFFFFFFFu, take)) {
+    const uint32_t takers = __ballot_sync(0xFFFFFFFFu, take);
+    taken += __popc(takers);
+    if (takers) {
       BvhNode nd = load_node(m.nodes, node);
       float dl = box_dist2(p, nd.l_lo, nd.l_hi), dr = box_dist2(p, nd.r_lo, nd.r_hi);
       uint32_t L = __float_as_uint(nd.l_lo.w), R = __float_as_uint(nd.l_hi.w);
       bool goL = take && dl <= best.d2, goR = take && dr <= best.d2;
+      if (goL) {
+        pill_raise(m.pills, 2u * node, nd.r_lo.w, p, ps, best.d2, &dl);
+        goL = dl <= best.d2;
+      }
+      if (goR) {
+        pill_raise(m.pills, 2u * node + 1u, nd.r_hi.w, p, ps, best.d2, &dr);
+        goR = dr <= best.d2;
+      }
       if (L & LEAF_BIT) {
         if (goL) eval(L & ~LEAF_BIT);
         goL = false;
       }
       if (R & LEAF_BIT) {
-        if (goR) eval(R & ~LEAF_BIT);
+        if (goR && dr <= best.d2) eval(R & ~LEAF_BIT);
         goR = false;
       }
       goL = goL && dl <= best.d2;
@@ -505,6 +557,7 @@ __device__ bool nearest_triangle_warp(const MeshView& m, P3 p, Nearest* io, uint
   // Non-negative d2 (or +inf / NaN-free boxes) order like their bits.
   unsigned long long best = nn_key(io->d2, io->tri);
   uint32_t best_leaf = io->leaf;
+  const float ps = pill_query_slack(p);
   int sp = 0;
   if (lane == 0) {
     s_node[0] = 0;
@@ -532,10 +585,14 @@ __device__ bool nearest_triangle_warp(const MeshView& m, P3 p, Nearest* io, uint
     if (node != 0xFFFFFFFFu && nd2 <= bound) {
       if constexpr (STATS) ++qc->visits;
       BvhNode nd = load_node(m.nodes, node);
+      // (with the node: a step's time is its chain of dependent loads)
+      const Pill pl[2] = {load_pill(m.pills, 2u * node), load_pill(m.pills, 2u * node + 1u)};
+      const float limit[2] = {nd.r_lo.w, nd.r_hi.w};
       const uint32_t ch[2] = {__float_as_uint(nd.l_lo.w), __float_as_uint(nd.l_hi.w)};
-      const float cd[2] = {box_dist2(p, nd.l_lo, nd.l_hi), box_dist2(p, nd.r_lo, nd.r_hi)};
+      float cd[2] = {box_dist2(p, nd.l_lo, nd.l_hi), box_dist2(p, nd.r_lo, nd.r_hi)};
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
+        if (cd[c] <= bound && bound < limit[c]) cd[c] = fmaxf(cd[c], pill_dist2(pl[c], p, ps));
         if (!(cd[c] <= bound)) continue;
         if (ch[c] & LEAF_BIT) {
           const uint32_t leaf = ch[c] & ~LEAF_BIT;
@@ -627,36 +684,22 @@ __device__ uint32_t ray_crossings(const MeshView& m, P3 o, bool* overflow, QCoun
   uint32_t stack[kStack];
   int sp = 0;
   uint32_t node = 0;
-  while (true) {
+  do {  // (one way back to the top: see nearest_triangle)
     if constexpr (STATS) ++qc->sign_visits;
     BvhNode nd = load_node(m.nodes, node);
     uint32_t L = __float_as_uint(nd.l_lo.w), R = __float_as_uint(nd.l_hi.w);
     bool goL = inside(nd.l_lo, nd.l_hi), goR = inside(nd.r_lo, nd.r_hi);
-    if (goL && (L & LEAF_BIT)) {
-      test(L & ~LEAF_BIT);
-      goL = false;
-    }
-    if (goR && (R & LEAF_BIT)) {
-      test(R & ~LEAF_BIT);
-      goR = false;
-    }
+    if (goL && (L & LEAF_BIT)) test(L & ~LEAF_BIT);
+    if (goR && (R & LEAF_BIT)) test(R & ~LEAF_BIT);
+    goL = goL && !(L & LEAF_BIT);
+    goR = goR && !(R & LEAF_BIT);
     if (goL && goR) {
       if (sp < kStack) stack[sp++] = R;
       else *overflow = true;
-      node = L;
-      continue;
     }
-    if (goL) {
-      node = L;
-      continue;
-    }
-    if (goR) {
-      node = R;
-      continue;
-    }
-    if (sp == 0) break;
-    node = stack[--sp];
-  }
+    node = goL ? L : (goR ? R : kNoNode);
+    if (node == kNoNode && sp > 0) node = stack[--sp];
+  } while (node != kNoNode);
   return count;
 }
 
@@ -808,6 +851,7 @@ __device__ float normal_band_fold(const MeshView& m, P3 p, float d2min, bool* na
   const double band = sqrt((double)d2min) * (1.0 + 1e-5) + 4e-6;
   const float reach = (float)((band + 2e-4) * (1.0 + 1e-6));
   const float reach2 = reach * reach;
+  const float ps = pill_query_slack(p);
   uint32_t c_idx[kBand];
   float c_d[kBand];
   int n = 0;
@@ -829,41 +873,28 @@ __device__ float normal_band_fold(const MeshView& m, P3 p, float d2min, bool* na
   } else {
     uint32_t stack[kStack];
     int sp = 0;
-    uint32_t node = 0;
-    uint32_t visits = 0;
-    while (true) {
-      if (++visits > budget) {
-        *finished = false;
-        return 0.0f;
-      }
+    uint32_t node = 0, visits = 0;
+    do {  // (one way back to the top: see nearest_triangle)
+      ++visits;
       if constexpr (STATS) ++qc->sign_visits;
       BvhNode nd = load_node(m.nodes, node);
       uint32_t L = __float_as_uint(nd.l_lo.w), R = __float_as_uint(nd.l_hi.w);
-      bool goL = box_dist2(p, nd.l_lo, nd.l_hi) <= reach2, goR = box_dist2(p, nd.r_lo, nd.r_hi) <= reach2;
-      if (goL && (L & LEAF_BIT)) {
-        consider(load_tri(m.stris, L & ~LEAF_BIT));
-        goL = false;
-      }
-      if (goR && (R & LEAF_BIT)) {
-        consider(load_tri(m.stris, R & ~LEAF_BIT));
-        goR = false;
-      }
+      float dl = box_dist2(p, nd.l_lo, nd.l_hi), dr = box_dist2(p, nd.r_lo, nd.r_hi);
+      pill_raise(m.pills, 2u * node, nd.r_lo.w, p, ps, reach2, &dl);
+      pill_raise(m.pills, 2u * node + 1u, nd.r_hi.w, p, ps, reach2, &dr);
+      if ((L & LEAF_BIT) && dl <= reach2) consider(load_tri(m.stris, L & ~LEAF_BIT));
+      if ((R & LEAF_BIT) && dr <= reach2) consider(load_tri(m.stris, R & ~LEAF_BIT));
+      const bool goL = !(L & LEAF_BIT) && dl <= reach2, goR = !(R & LEAF_BIT) && dr <= reach2;
       if (goL && goR) {
         if (sp < kStack) stack[sp++] = R;
         else *overflow = true;
-        node = L;
-        continue;
       }
-      if (goL) {
-        node = L;
-        continue;
-      }
-      if (goR) {
-        node = R;
-        continue;
-      }
-      if (sp == 0) break;
-      node = stack[--sp];
+      node = goL ? L : (goR ? R : kNoNode);
+      if (node == kNoNode && sp > 0) node = stack[--sp];
+    } while (node != kNoNode && visits < budget);
+    if (node != kNoNode) {
+      *finished = false;
+      return 0.0f;
     }
   }
   float best = F32_MAX;
@@ -909,6 +940,7 @@ __device__ bool normal_band_fold_warp(const MeshView& m, P3 p, float d2min, uint
   const double band = sqrt((double)d2min) * (1.0 + 1e-5) + 4e-6;
   const float reach = (float)((band + 2e-4) * (1.0 + 1e-6));
   const float reach2 = reach * reach;
+  const float ps = pill_query_slack(p);
   if (lane == 0) *s_count = 0;
   __syncwarp();
   bool over = false;
@@ -941,11 +973,14 @@ __device__ bool normal_band_fold_warp(const MeshView& m, P3 p, float d2min, uint
       if (node != 0xFFFFFFFFu) {
         if constexpr (STATS) ++qc->sign_visits;
         const BvhNode nd = load_node(m.nodes, node);
+        const Pill pl[2] = {load_pill(m.pills, 2u * node), load_pill(m.pills, 2u * node + 1u)};
+        const float limit[2] = {nd.r_lo.w, nd.r_hi.w};
         const uint32_t ch[2] = {__float_as_uint(nd.l_lo.w), __float_as_uint(nd.l_hi.w)};
-        const bool go[2] = {box_dist2(p, nd.l_lo, nd.l_hi) <= reach2, box_dist2(p, nd.r_lo, nd.r_hi) <= reach2};
+        float cd[2] = {box_dist2(p, nd.l_lo, nd.l_hi), box_dist2(p, nd.r_lo, nd.r_hi)};
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          if (!go[c]) continue;
+          if (cd[c] <= reach2 && reach2 < limit[c]) cd[c] = fmaxf(cd[c], pill_dist2(pl[c], p, ps));
+          if (!(cd[c] <= reach2)) continue;
           if (ch[c] & LEAF_BIT) consider(ch[c] & ~LEAF_BIT);
           else push[npush++] = ch[c];
         }
@@ -1238,17 +1273,15 @@ __global__ void k_query_keys(const float* __restrict__ q, uint64_t nq, MeshView 
 // Node-visit budget of the single-thread search (0: single pass only).
 std::atomic<uint32_t> g_query_budget{768};
 
-// Batch size from which Raycast, Rtree and vector queries search a warp at a
-// time (measured crossover: star s6 and the 512^2 terrain are even at 400k to
-// 600k queries; 1M star points 8.0 -> 7.1 ms, 4M terrain points 15.2 -> 10.7 ms;
-// 100k star points 2.4 -> 2.9 ms).
-constexpr uint64_t kPacketMinQueries = 1u << 19;
-// Batches up to this many queries run one warp per query (k_query_warpwise).
-// Measured on B200, star s6, RtreeBvh / Rtree, against the two-pass path:
-// 1,000 queries 0.39 / 0.37 ms against 0.57 / 0.45 ms, 4,000 0.43 / 0.39
-// against 0.60 / 0.46 ms, but 16,000 1.24 / 1.13 against 0.98 / 0.74 ms
-// (bit-identical results throughout).
-constexpr uint64_t kWarpwiseMaxQueries = 8192;
+// Batches up to this many queries run one warp per query (k_query_warpwise), on
+// meshes of up to kWarpwiseSmallMesh triangles and on larger ones, whose
+// searches fill the warp's lanes for longer.  Measured on B200 against the
+// two-pass path: 10,000 queries on star s3 (1,280 triangles) 0.12 against 0.15
+// ms, s5 (20,480) 0.22 / 0.22; s6 (81,920) 4,000 queries 0.19 against 0.23 ms,
+// 6,000 0.26 / 0.25, the terrain strip (524,282) 0.14 / 0.15 and 0.21 / 0.16
+// (bit-identical throughout).
+constexpr uint64_t kWarpwiseMaxQueries = 10240, kWarpwiseMaxLarge = 4096;
+constexpr uint32_t kWarpwiseSmallMesh = 1u << 15;
 constexpr uint64_t kMortonMinQueries = 1u << 17;  // batch size from which queries run in Morton order
 
 namespace {
@@ -1401,7 +1434,7 @@ int query_points(const MeshView& m, int accel, int sign, const float* d_q, uint6
                                 ? Q_RTREE
                                 : ((accel == M2S_ACCEL_BVH && sign == M2S_SIGN_NORMAL) ? Q_BVH_NORMAL : Q_BVH_RAYCAST));
   // Small batches (a mesh of more than one triangle): one warp per query.
-  if (nq <= kWarpwiseMaxQueries && !(m.root & LEAF_BIT)) {
+  if (nq <= (m.n_tris <= kWarpwiseSmallMesh ? kWarpwiseMaxQueries : kWarpwiseMaxLarge) && !(m.root & LEAF_BIT)) {
     const bool counting = profiling_enabled() || grid_tuning().fp64_audit;
     DevBuf<unsigned long long> qs;
     int st;
@@ -1438,15 +1471,14 @@ int query_points(const MeshView& m, int accel, int sign, const float* d_q, uint6
     }
     return M2S_OK;
   }
-  // Morton-ordered launch for large batches: from 2^17 queries (below, the
-  // sort's launches cost more than coherent warps save: 10k RtreeBvh points
-  // on icosphere s3 0.33 -> 0.21 ms unsorted, star s6 50k 1.84 -> 1.65 ms; at
-  // 200k sorting wins, 3.75 -> 3.20 ms), and from 4096 for Bvh(Normal), whose
-  // packet search needs the order.
+  // Morton-ordered launch for large batches, whose warps start their searches
+  // together: from 2^17 queries; below, the sort's launches cost more than
+  // coherent warps save (10k RtreeBvh points on icosphere s3 0.33 -> 0.21 ms
+  // unsorted; Bvh(Normal) at 20,000 points on star s6 0.69 -> 0.43 ms).
   DevBuf<uint32_t> keys, order;
   const uint32_t* ord = nullptr;
   int st;
-  if (nq >= (mode == Q_BVH_NORMAL ? 4096u : kMortonMinQueries)) {
+  if (nq >= kMortonMinQueries) {
     if ((st = keys.alloc(nq, s)) || (st = order.alloc(nq, s))) return st;
     k_query_keys<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(d_q, nq, m, keys.p, order.p);
     M2S_CUDA(cudaGetLastError());
@@ -1459,22 +1491,8 @@ int query_points(const MeshView& m, int accel, int sign, const float* d_q, uint6
   DevBuf<uint32_t> hard_count;
   const uint32_t base_budget =
       budget_override >= 0 ? (uint32_t)budget_override : g_query_budget.load(std::memory_order_relaxed);
-  // Bvh(Normal) hands long searches and tie-band folds to the warp pass in
-  // batches below 2^18 queries (where the budget is base / 16), whose
-  // single-thread band traversals set the time (star s6: 1,000 points 6.17
-  // -> 0.59 ms, 10,000 15.5 -> 1.4 ms, 131,072 21.9 -> 3.4 ms, 262,143 23.9
-  // -> 5.2 ms; star s4 200,000 4.1 -> 1.9 ms; the terrain strip: 20,000 3.69
-  // -> 1.39 ms, 131,072 2.85 -> 2.38 ms, though 262,143 3.36 -> 4.31 ms);
-  // from there on the one-pass packet search keeps its coherence and wins on
-  // the terrain (400,000 points 4.1 against 9.0 ms with the hand-off at the
-  // default budget, 1M 6.7 against 20.0) and ties on the star (1M 30.2
-  // against 30.7 ms).  A base budget of at most kNormalHandoffMaxBudget keeps
-  // the hand-off at every size, which suits closed meshes whose deep-interior
-  // points make long searches (star s6 at budget 64: 400,000 points 27.5 ->
-  // 7.7 ms, 1M 29.8 -> 17.0 ms) but not open ones (the terrain: 4.1 -> 6.3
-  // and 6.6 -> 14.7 ms); the autotuner tries it.
-  const bool two_pass =
-      base_budget > 0 && (mode != Q_BVH_NORMAL || nq < (1u << 18) || base_budget <= kNormalHandoffMaxBudget);
+  // Bvh(Normal) hands long tie-band folds to the warp pass too.
+  const bool two_pass = base_budget > 0;
   if (two_pass) {
     if ((st = hard.alloc(nq, s)) || (st = hard_count.alloc(1, s))) return st;
     M2S_CUDA(cudaMemsetAsync(hard_count.p, 0, 4, s));
@@ -1492,10 +1510,8 @@ int query_points(const MeshView& m, int accel, int sign, const float* d_q, uint6
     if ((st = qs.alloc(kQueryCounters, s))) return st;
     M2S_CUDA(cudaMemsetAsync(qs.p, 0, 8 * kQueryCounters, s));
   }
-  // Morton-ordered warps search together (nearest_triangle_packet): always
-  // for Bvh(Normal), and for the others from kPacketMinQueries on, where
-  // throughput rather than the longest warp sets the time.
-  const bool packet = ord != nullptr && (mode == Q_BVH_NORMAL || nq >= kPacketMinQueries);
+  // Morton-ordered warps search together for as long as that pays (nearest_triangle_packet).
+  const bool packet = ord != nullptr;
   if (counting)
     launch_queries<true>(mode, m, d_q, ord, nq, d_out, d_vec, d_inside, d_status, budget, hp, hc, two_pass, packet,
                          blocks, qs.p, s);

@@ -84,10 +84,10 @@ struct MeshEntry {
 };
 
 // Device bytes a resident mesh holds: triangle records in both orders (48 B
-// each) and 64-byte LBVH nodes; the build needs about as much again for a
+// each), 64-byte LBVH nodes and 64 bytes of pillboxes a node; the build needs about as much again for a
 // moment (vertices, indices, Morton keys, sort buffers).
 uint64_t mesh_bytes(uint64_t tris, int accel) {
-  return accel == M2S_ACCEL_NONE ? 48 * tris : 160 * tris;
+  return accel == M2S_ACCEL_NONE ? 48 * tris : 224 * tris;
 }
 uint64_t upload_bytes(uint64_t tris, uint64_t nv, uint64_t ni, int bits, int accel) {
   return 2 * mesh_bytes(tris, accel) + 12 * nv + ni * (bits / 8) + (1u << 20);
