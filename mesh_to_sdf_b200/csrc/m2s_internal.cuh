@@ -149,11 +149,15 @@ struct DeviceMesh {
 int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, cudaStream_t s,
                       bool with_tree = true);
 
-// Stable LSD radix sort of (key, value) pairs over the low key_bits bits.
-int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, cudaStream_t s);
+// ---- sorting (m2s_sort.cu) ----------------------------------------------------
 
-// Exclusive scan of n uint32 (in place allowed); returns the total via *d_total if non-null.
-int exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* d_total, cudaStream_t s);
+// Stable LSD radix sort of (key, value) pairs over the low key_bits bits.
+// keep_keys = false leaves the keys in no order (the values alone are wanted).
+int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, cudaStream_t s, bool keep_keys = true);
+
+// order: 0 .. n - 1 stably by f32::total_cmp of d; minmax (2 floats, may be
+// NULL): the extremes of the values that are no NaN.
+int sort_floats(const float* d, uint64_t n, uint32_t* order, float* minmax, cudaStream_t s);
 
 // ---- point queries (m2s_query.cu) -------------------------------------------
 

@@ -1,5 +1,5 @@
-// LBVH build on the device: triangle records, Morton codes, a stable LSD
-// radix sort, Karras (2012) binary radix tree emission and a bottom-up refit.
+// LBVH build on the device: triangle records, Morton codes sorted (m2s_sort.cu),
+// Karras (2012) binary radix tree emission, a bottom-up refit and pillboxes.
 //
 // The tree replaces the bvh 0.10 / rstar 0.12 trees of the Rust crate
 // (generate/generic/bvh.rs:230-254, rtree.rs:279-304, rtree_bvh.rs:100-141,
@@ -118,150 +118,6 @@ __global__ void k_morton(const float4* __restrict__ boxes, uint64_t n, const uin
   }
   keys[t] = (spread10(q[0]) << 2) | (spread10(q[1]) << 1) | spread10(q[2]);
   vals[t] = (uint32_t)t;
-}
-
-// ---- exclusive scan (u32) --------------------------------------------------
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kThreads * kScanItems;
-
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total) {
-  __shared__ uint32_t warp_sums[kThreads / 32];
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) warp_sums[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t s = lane < kThreads / 32 ? warp_sums[lane] : 0;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xFFFFFFFFu, s, o);
-      if (lane >= o) s += y;
-    }
-    if (lane < kThreads / 32) warp_sums[lane] = s;
-  }
-  __syncthreads();
-  uint32_t prefix = warp ? warp_sums[warp - 1] : 0;
-  *total = warp_sums[kThreads / 32 - 1];
-  __syncthreads();
-  return prefix + x - v;
-}
-
-__global__ void k_scan_tiles(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* tile_sums) {
-  uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-  uint32_t v[kScanItems], s = 0;
-  for (int k = 0; k < kScanItems; ++k) {
-    v[k] = base + k < n ? in[base + k] : 0;
-    s += v[k];
-  }
-  uint32_t total;
-  uint32_t ex = block_exclusive_scan(s, &total);
-  for (int k = 0; k < kScanItems; ++k) {
-    if (base + k < n) out[base + k] = ex;
-    ex += v[k];
-  }
-  if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-__global__ void k_add_tiles(uint32_t* out, uint64_t n, const uint32_t* tile_offsets) {
-  uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-  uint32_t add = tile_offsets[blockIdx.x];
-  for (int k = 0; k < kScanItems; ++k)
-    if (base + k < n) out[base + k] += add;
-}
-
-// total = last exclusive prefix + last input (saved before an in-place scan).
-__global__ void k_copy_total(const uint32_t* scanned, uint64_t n, const uint32_t* last_in, uint32_t* total) {
-  *total = scanned[n - 1] + *last_in;
-}
-
-// ---- radix sort ------------------------------------------------------------
-constexpr int kSortItems = 8;
-constexpr int kSortTile = kThreads * kSortItems;
-constexpr int kDigits = 256;
-
-__global__ void k_hist(const uint32_t* __restrict__ keys, uint64_t n, int shift, uint32_t* hist, uint32_t nblocks) {
-  __shared__ uint32_t h[kDigits];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  uint64_t base = (uint64_t)blockIdx.x * kSortTile;
-  for (int it = 0; it < kSortItems; ++it) {
-    uint64_t k = base + (uint64_t)it * kThreads + threadIdx.x;
-    if (k < n) atomicAdd(&h[(keys[k] >> shift) & 0xFFu], 1u);
-  }
-  __syncthreads();
-  hist[(uint64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
-}
-
-// Stable scatter: within a tile, keys keep their input order per digit.  The
-// tile is first ordered by digit in shared memory (a key's place: the tile's
-// start of its digit, from the scanned offsets, plus the same-digit keys
-// before it), then each digit's run is written out contiguously, so
-// neighbouring threads write neighbouring addresses.
-__global__ void k_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* kout,
-                          uint32_t* vout, uint64_t n, int shift, const uint32_t* offsets, uint32_t nblocks) {
-  __shared__ uint32_t run[kDigits];
-  __shared__ uint32_t wcnt[kThreads / 32][kDigits];
-  __shared__ uint32_t base_off[kDigits];
-  __shared__ uint32_t tile_start[kDigits];
-  __shared__ uint32_t s_key[kSortTile], s_val[kSortTile];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
-  const uint32_t tile_n = (uint32_t)(n - base < (uint64_t)kSortTile ? n - base : (uint64_t)kSortTile);
-  {
-    // this tile's count of digit d: the next offset (digit-major) minus its own
-    const uint64_t idx = (uint64_t)threadIdx.x * nblocks + blockIdx.x;
-    const uint32_t off = offsets[idx];
-    const uint32_t next = idx + 1 < (uint64_t)kDigits * nblocks ? offsets[idx + 1] : (uint32_t)n;
-    base_off[threadIdx.x] = off;
-    // exclusive scan of the counts over the 256 digits (one per thread)
-    uint32_t c = next - off, incl = c;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane == 31) wcnt[0][warp] = incl;
-    __syncthreads();
-    uint32_t wbase = 0;
-    for (int w = 0; w < warp; ++w) wbase += wcnt[0][w];
-    tile_start[threadIdx.x] = wbase + incl - c;
-    run[threadIdx.x] = 0;
-    __syncthreads();
-  }
-  const uint32_t lt_mask = (1u << lane) - 1u;
-  for (int it = 0; it < kSortItems; ++it) {
-    for (int w = 0; w < kThreads / 32; ++w) wcnt[w][threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t t = (uint32_t)it * kThreads + threadIdx.x;
-    const bool valid = t < tile_n;
-    const uint32_t key = valid ? kin[base + t] : 0, val = valid ? vin[base + t] : 0;
-    const uint32_t digit = valid ? (key >> shift) & 0xFFu : 0x100u;
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, digit);
-    const uint32_t lrank = __popc(peers & lt_mask);
-    if (valid && lrank == 0) wcnt[warp][digit] = __popc(peers);
-    __syncthreads();
-    if (valid) {
-      uint32_t before = run[digit];
-      for (int w = 0; w < warp; ++w) before += wcnt[w][digit];
-      const uint32_t pos = tile_start[digit] + before + lrank;  // < tile_n
-      s_key[pos] = key;
-      s_val[pos] = val;
-    }
-    __syncthreads();
-    uint32_t add = 0;
-    for (int w = 0; w < kThreads / 32; ++w) add += wcnt[w][threadIdx.x];
-    run[threadIdx.x] += add;
-    __syncthreads();
-  }
-  for (uint32_t t = threadIdx.x; t < tile_n; t += kThreads) {
-    const uint32_t key = s_key[t];
-    const uint32_t d = (key >> shift) & 0xFFu;
-    const uint32_t dst = base_off[d] + (t - tile_start[d]);
-    kout[dst] = key;
-    vout[dst] = s_val[t];
-  }
 }
 
 // ---- Karras hierarchy --------------------------------------------------------
@@ -493,61 +349,6 @@ __global__ void k_pills(const TriRec* __restrict__ stris, BvhNode* __restrict__ 
 inline unsigned grid_for(uint64_t n, int threads = kThreads) { return (unsigned)((n + threads - 1) / threads); }
 
 }  // namespace
-
-int exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, uint32_t* d_total, cudaStream_t s) {
-  if (n == 0) {
-    if (d_total) M2S_CUDA(cudaMemsetAsync(d_total, 0, 4, s));
-    return M2S_OK;
-  }
-  uint64_t tiles = (n + kScanTile - 1) / kScanTile;
-  DevBuf<uint32_t> sums;
-  int st = sums.alloc(tiles + 1, s);
-  if (st) return st;
-  // The last input is needed for the total if the scan runs in place.
-  DevBuf<uint32_t> last;
-  if (d_total) {
-    if ((st = last.alloc(1, s))) return st;
-    M2S_CUDA(cudaMemcpyAsync(last.p, in + n - 1, 4, cudaMemcpyDeviceToDevice, s));
-  }
-  k_scan_tiles<<<(unsigned)tiles, kThreads, 0, s>>>(in, out, n, sums.p);
-  M2S_CUDA(cudaGetLastError());
-  if (tiles > 1) {
-    if ((st = exclusive_scan_u32(sums.p, sums.p, tiles, nullptr, s))) return st;
-    k_add_tiles<<<(unsigned)tiles, kThreads, 0, s>>>(out, n, sums.p);
-    M2S_CUDA(cudaGetLastError());
-  }
-  if (d_total) {
-    k_copy_total<<<1, 1, 0, s>>>(out, n, last.p, d_total);
-    M2S_CUDA(cudaGetLastError());
-  }
-  return M2S_OK;
-}
-
-int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, cudaStream_t s) {
-  if (n <= 1) return M2S_OK;
-  if (key_bits <= 0 || key_bits > 32 || n > 0xFFFFFFFFull) return M2S_ERR_INVALID_ARGUMENT;
-  uint32_t nblocks = (uint32_t)((n + kSortTile - 1) / kSortTile);
-  DevBuf<uint32_t> k2, v2, hist;
-  int st;
-  if ((st = k2.alloc(n, s)) || (st = v2.alloc(n, s)) || (st = hist.alloc((uint64_t)kDigits * nblocks, s))) return st;
-  uint32_t *ka = keys, *va = vals, *kb = k2.p, *vb = v2.p;
-  int passes = (key_bits + 7) / 8;
-  for (int p = 0; p < passes; ++p) {
-    int shift = 8 * p;
-    k_hist<<<nblocks, kThreads, 0, s>>>(ka, n, shift, hist.p, nblocks);
-    M2S_CUDA(cudaGetLastError());
-    if ((st = exclusive_scan_u32(hist.p, hist.p, (uint64_t)kDigits * nblocks, nullptr, s))) return st;
-    k_scatter<<<nblocks, kThreads, 0, s>>>(ka, va, kb, vb, n, shift, hist.p, nblocks);
-    M2S_CUDA(cudaGetLastError());
-    std::swap(ka, kb);
-    std::swap(va, vb);
-  }
-  if (ka != keys) {
-    M2S_CUDA(cudaMemcpyAsync(keys, ka, n * 4, cudaMemcpyDeviceToDevice, s));
-    M2S_CUDA(cudaMemcpyAsync(vals, va, n * 4, cudaMemcpyDeviceToDevice, s));
-  }
-  return M2S_OK;
-}
 
 int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, cudaStream_t s, bool with_tree) {
   if (in.n_tris > 0x7FFFFFFFull) return M2S_ERR_INVALID_ARGUMENT;

@@ -1353,7 +1353,7 @@ int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, 
     k_bf_bounds<<<(unsigned)std::min<uint64_t>((nq + 255) / 256, 148u * 8u), 256, 0, s>>>(d_q, nq, bounds.p);
     k_bf_keys<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(d_q, nq, bounds.p, keys.p, order.p);
     M2S_CUDA(cudaGetLastError());
-    if ((st = radix_sort_pairs(keys.p, order.p, nq, 30, s))) return st;
+    if ((st = radix_sort_pairs(keys.p, order.p, nq, 30, s, /*keep_keys=*/false))) return st;
     ord = order.p;
   }
   if (sign == M2S_SIGN_RAYCAST) {
@@ -1482,7 +1482,7 @@ int query_points(const MeshView& m, int accel, int sign, const float* d_q, uint6
     if ((st = keys.alloc(nq, s)) || (st = order.alloc(nq, s))) return st;
     k_query_keys<<<(unsigned)((nq + 255) / 256), 256, 0, s>>>(d_q, nq, m, keys.p, order.p);
     M2S_CUDA(cudaGetLastError());
-    if ((st = radix_sort_pairs(keys.p, order.p, nq, 30, s))) return st;
+    if ((st = radix_sort_pairs(keys.p, order.p, nq, 30, s, /*keep_keys=*/false))) return st;
     ord = order.p;
   }
   unsigned blocks = (unsigned)((nq + 127) / 128);
