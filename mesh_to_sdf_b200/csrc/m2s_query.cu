@@ -1,10 +1,10 @@
 // Point queries: generate_sdf / query_sdf for every AccelerationMethod.
 //
-//  * None  (generate/generic/default.rs:22-85): k_brute — every query against
+//  * None  (generate/generic/default.rs:22-85): k_brute_* — every query against
 //    every triangle.  Triangle tiles are staged in shared memory by the bulk
-//    copy engine (cp.async.bulk + mbarrier, double-buffered); each thread owns
-//    one query and folds the tile in triangle order, exactly the reference's
-//    fold order; batches of 2^28 pairs or more are visited in Morton order.
+//    copy engine (cp.async.bulk + mbarrier, double-buffered); a thread owns two
+//    queries (Raycast) or one (Normal, folded in triangle order, exactly the
+//    reference's fold order); batches of 2^24 pairs or more are visited in Morton order.
 //    Normal batches of fewer than 2^17 queries take k_brute_normal_warp: a
 //    warp per query, the same fold in the same order.
 //  * Bvh(Raycast) / RtreeBvh (bvh.rs:104-180, rtree_bvh.rs:143-201): exact
@@ -29,6 +29,9 @@ namespace {
 
 constexpr float F32_MAX = 3.40282347e+38f;
 
+__device__ __forceinline__ float pill_query_slack(P3 p) {
+  return kPillSlack * fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z)));
+}
 __device__ __forceinline__ P3 load_query(const float* q, uint64_t i) { return {q[3 * i], q[3 * i + 1], q[3 * i + 2]}; }
 
 // ---------------------------------------------------------------------------
@@ -36,39 +39,266 @@ __device__ __forceinline__ P3 load_query(const float* q, uint64_t i) { return {q
 constexpr int kBfThreads = 128;
 constexpr int kBfTile = 256;  // triangles per stage: 256 * 48 B = 12 KiB
 
-// Raycast splits the triangle range into gridDim.y chunks (min and hit parity
-// commute): each chunk folds its part and merges into `part` (atomicMin on the
-// squared distance bits, atomicXor on the parity).  Normal folds all
-// triangles in order in one chunk (compare_distances ties depend on order).
+// Raycast: two queries per thread, their arithmetic packed as f32x2 (one
+// instruction for both, each half rounded like the scalar one), so a warp
+// holds 64 queries.  The kernel is bound by instruction issue: of a pair's
+// work only the three edge functions of the +X ray test are needed for every
+// triangle (15 of the 60 scalar instructions a pair took; the triangle's share
+// of the test, its edges, is formed once per tile), and the plane bound.
 //
-// Raycast: a triangle whose plane bound (tri_plane in m2s_geo.cuh) exceeds
-// the query's best distance so far cannot lower the minimum, so its closest
-// point is not evaluated; its +X ray test always is (the parity counts every
-// triangle).  Rust's f32::min ignores a NaN distance (default.rs:58), so a
-// skipped triangle changes nothing even then.  The planes of a tile are
-// formed in shared memory as it lands.
-template <int SIGN>
-__global__ void __launch_bounds__(kBfThreads) k_brute(const TriRec* __restrict__ tris, uint32_t T,
-                                                      const float* __restrict__ q, uint64_t nq,
-                                                      float* __restrict__ out, uint32_t* status,
-                                                      uint2* __restrict__ part, const uint32_t* __restrict__ order) {
+// The triangle range is split into gridDim.y chunks (min and hit parity
+// commute): each chunk folds its part and merges into `part` (atomicMin on the
+// squared distance bits, atomicXor on the parity).
+//
+// A triangle whose plane bound (tri_plane in m2s_geo.cuh) exceeds the query's
+// best distance so far cannot lower the minimum, so its closest point is not
+// evaluated; its ray test always is (the parity counts every triangle).  Where
+// the plane comes near (a third of the planes of a closed mesh, for a point
+// outside it), the disc around the triangle decides in the same way: the bound
+// of Pill (m2s_internal.cuh) with a single triangle, for triangles whose angle
+// at a has sin^2 >= 1/200 as for the plane.  Below the reach the reference's
+// point leaves the disc by less than the slack, and at up to 2^8.5 times the
+// reach it errs by less than a fifth of the distance, so the triangle is still
+// the farther one; beyond that the disc says nothing.
+// Rust's f32::min ignores a NaN distance (default.rs:58), so a skipped
+// triangle changes nothing even then.
+//
+// Measured (star s6, 65,536 points, 5.4G pairs): 14.1 ms with one query a
+// thread, 10.2 packed, 9.4 with the disc, 8.7 with one branch for the usual
+// case, 7.7 (697 G pairs/s) with blocks of 256 that share a tile (four of them
+// an SM; 128: 8.6, 512: 7.6).  Tiles of 64 rather than 128 triangles cost 1 %
+// there and let small meshes spread over more blocks (1,280 triangles, 1,000
+// points 0.125 -> 0.082 ms).
+constexpr int kBrThreads = 256;
+constexpr int kBrTile = 64;  // triangles per stage
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  return ((f32x2)__float_as_uint(hi) << 32) | __float_as_uint(lo);
+}
+__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// a - b, rounded once: b * -1 is exact.
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, pack2(-1.0f, -1.0f), a); }
+// Sign bit set when the three do not all have the same one.
+__device__ __forceinline__ uint32_t mixed_sign(float a, float b, float c) {
+  const uint32_t x = __float_as_uint(a), y = __float_as_uint(b), z = __float_as_uint(c);
+  return (x ^ y) | (y ^ z);
+}
+
+// A triangle as the pair loop reads it, every value twice (one for each
+// query): for the edges t1 t2, t2 t0, t0 t1 of ray_hit_aligned<0> the
+// first vertex's -y, -z and the edge's y, z; the plane's unit normal and
+// offset, scaled by the bound's 1 - 2^-13, and its slack.
+struct __align__(16) BrutePair {
+  ulonglong2 edge[3][2];  // (-y, -z), (ey, ez)
+  ulonglong2 nxy, nzw;
+  f32x2 slack;
+  float disc_slack, disc_limit2;  // of the disc: h's slack; squared reach (0: none)
+  ulonglong2 cxy, czr;            // its centre, its radius with the slack
+};
+
+__global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* __restrict__ tris, uint32_t T,
+                                                              const float* __restrict__ q, uint64_t nq,
+                                                              float* __restrict__ out, uint32_t* status,
+                                                              uint2* __restrict__ part,
+                                                              const uint32_t* __restrict__ order) {
+  __shared__ __align__(128) TriRec tile[2][kBrTile];
+  __shared__ BrutePair pair[kBrTile];
+  __shared__ __align__(8) uint64_t bar[2];
+  const int tid = threadIdx.x;
+  uint64_t qi[2];
+  P3 p[2];
+  bool valid[2];
+  for (int u = 0; u < 2; ++u) {  // neighbours in Morton order share a warp
+    const uint64_t k = ((uint64_t)blockIdx.x * kBrThreads + tid) * 2 + u;
+    valid[u] = k < nq;
+    qi[u] = valid[u] && order ? order[k] : k;
+    p[u] = valid[u] ? load_query(q, qi[u]) : P3{0.0f, 0.0f, 0.0f};
+  }
+  const f32x2 px = pack2(p[0].x, p[1].x), py = pack2(p[0].y, p[1].y), pz = pack2(p[0].z, p[1].z);
+  // this block's chunk of triangles: whole tiles [t_begin, t_end)
+  const uint32_t all_tiles = (T + kBrTile - 1) / kBrTile;
+  const uint32_t per = (all_tiles + gridDim.y - 1) / gridDim.y;
+  const uint32_t t_begin = min(all_tiles, blockIdx.y * per), t_end = min(all_tiles, t_begin + per);
+  const uint32_t ntile = t_end - t_begin;
+  tris += (uint64_t)t_begin * kBrTile;
+  T = ntile == 0 ? 0u : (t_end == all_tiles ? T - t_begin * kBrTile : ntile * kBrTile);
+
+  if (tid == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  auto issue = [&](uint32_t i) {
+    uint32_t cnt = min((uint32_t)kBrTile, T - i * kBrTile);
+    uint32_t bytes = cnt * (uint32_t)sizeof(TriRec);
+    mbar_arrive_expect_tx(&bar[i & 1], bytes);
+    bulk_g2s(&tile[i & 1][0], tris + (uint64_t)i * kBrTile, bytes, &bar[i & 1]);
+  };
+  if (tid == 0) {
+    if (ntile > 0) issue(0);
+    if (ntile > 1) issue(1);
+  }
+
+  float best[2] = {INFINITY, INFINITY};  // squared distances
+  // A plane's |h| must exceed its slack plus `above` to skip the triangle: the
+  // query's best distance and its share of the slack.
+  const float pslack[2] = {plane_query_slack(p[0]), plane_query_slack(p[1])};
+  const float dslack[2] = {pill_query_slack(p[0]), pill_query_slack(p[1])};
+  f32x2 above = pack2(INFINITY, INFINITY);
+  uint32_t hits[2] = {0u, 0u};
+  bool lost = false;
+  for (uint32_t i = 0; i < ntile; ++i) {
+    const int buf = i & 1;
+    if (!mbar_wait_bounded(&bar[buf], (i >> 1) & 1)) lost = true;
+    const uint32_t cnt = min((uint32_t)kBrTile, T - i * kBrTile);
+    const TriRec* tl = tile[buf];
+    lost = __syncthreads_or(lost);  // pairs are only formed from a tile every thread has
+    if (!lost && tid < (int)cnt) {
+      const P3 t0 = p3(tl[tid].a), t1 = p3(tl[tid].b), t2 = p3(tl[tid].c);
+      auto twice = [](float v, float w) { return make_ulonglong2(pack2(v, v), pack2(w, w)); };
+      auto edge = [&](P3 s, P3 e, int k) {
+        pair[tid].edge[k][0] = twice(-s.y, -s.z);
+        pair[tid].edge[k][1] = twice(fs(e.y, s.y), fs(e.z, s.z));
+      };
+      edge(t1, t2, 0);
+      edge(t2, t0, 1);
+      edge(t0, t1, 2);
+      const TriPlane pl = tri_plane(t0, t1, t2, __float_as_int(tl[tid].a.w));
+      const float c = 1.0f - 0x1p-13f;
+      pair[tid].nxy = twice(pl.n.x * c, pl.n.y * c);
+      pair[tid].nzw = twice(pl.n.z * c, -pl.n.w * c);
+      pair[tid].slack = pack2(pl.slack, pl.slack);
+      const float cx = (t0.x + t1.x + t2.x) * (1.0f / 3.0f), cy = (t0.y + t1.y + t2.y) * (1.0f / 3.0f),
+                  cz = (t0.z + t1.z + t2.z) * (1.0f / 3.0f);
+      auto len2 = [](P3 u, float x, float y, float z) {
+        return (u.x - x) * (u.x - x) + (u.y - y) * (u.y - y) + (u.z - z) * (u.z - z);
+      };
+      const float r2 = fmaxf(len2(t0, cx, cy, cz), fmaxf(len2(t1, cx, cy, cz), len2(t2, cx, cy, cz)));
+      const float e0 = len2(t0, t1.x, t1.y, t1.z), e1 = len2(t1, t2.x, t2.y, t2.z), e2 = len2(t2, t0.x, t0.y, t0.z);
+      const P3 w = vcross(vsub(t1, t0), vsub(t2, t0));
+      const float reach = kPillReach * sqrtf(w.x * w.x + w.y * w.y + w.z * w.z) * sqrtf(fminf(e0, fminf(e1, e2))) /
+                          fmaxf(e0, fmaxf(e1, e2));
+      const float slack = pl.slack * (kPillSlack / 0x1p-11f);  // the plane's is 2^-11 of the magnitude
+      pair[tid].disc_slack = slack;
+      pair[tid].disc_limit2 = pl.slack < INFINITY && reach > 0.0f ? fminf(reach * reach, 0x1p100f) : 0.0f;
+      const float r = sqrtf(r2) * 1.00001f + slack;
+      pair[tid].cxy = twice(-cx, -cy);
+      pair[tid].czr = twice(-cz, r);
+    }
+    __syncthreads();
+    if (!lost) {
+#pragma unroll 2
+      for (uint32_t j = 0; j < cnt; ++j) {
+        const BrutePair& t = pair[j];
+        f32x2 w[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const ulonglong2 v = t.edge[k][0], e = t.edge[k][1];
+          w[k] = sub2(mul2(add2(pz, v.y), e.x), mul2(add2(py, v.x), e.y));
+        }
+        const ulonglong2 nxy = t.nxy, nzw = t.nzw;
+        const f32x2 h = fma2(nxy.x, px, fma2(nxy.y, py, fma2(nzw.x, pz, nzw.y)));
+        const f32x2 reach = add2(above, t.slack);
+        // A crossing's edge functions have one sign; the exact test follows.
+        const uint32_t mixed0 = mixed_sign(lo2(w[0]), lo2(w[1]), lo2(w[2]));
+        const uint32_t mixed1 = mixed_sign(hi2(w[0]), hi2(w[1]), hi2(w[2]));
+        bool near0 = !(fabsf(lo2(h)) > lo2(reach)), near1 = !(fabsf(hi2(h)) > hi2(reach));
+        if ((int)(mixed0 & mixed1) < 0 && !near0 && !near1) continue;  // the usual case, in one branch
+        if ((int)mixed0 >= 0 || (int)mixed1 >= 0) {  // default.rs:59-62
+          const P3 a = p3(tl[j].a), b = p3(tl[j].b), c = p3(tl[j].c);
+          float tt;
+          if ((int)mixed0 >= 0) hits[0] += ray_hit_aligned<0>(p[0], a, b, c, &tt) ? 1u : 0u;
+          if ((int)mixed1 >= 0) hits[1] += ray_hit_aligned<0>(p[1], a, b, c, &tt) ? 1u : 0u;
+        }
+        if (near0 || near1) {
+          const ulonglong2 cxy = t.cxy, czr = t.czr;
+          const f32x2 x = add2(px, cxy.x), y = add2(py, cxy.y), z = add2(pz, czr.x);
+          const f32x2 a = fma2(nxy.x, x, fma2(nxy.y, y, mul2(nzw.x, z)));  // no more than the distance along n
+          const f32x2 qq = fma2(x, x, fma2(y, y, mul2(z, z)));
+          auto farther = [&](float a1, float q2, float r, float ps, float best2) {
+            const float up = a1 * (1.0f + 0x1p-12f);  // no less than it
+            float l;
+            asm("sqrt.approx.f32 %0, %1;" : "=f"(l) : "f"(fmaxf(fmaf(-up, up, q2 * (1.0f - 0x1p-20f)), 0.0f)));
+            const float da = fmaxf(fabsf(a1) - (t.disc_slack + ps), 0.0f), dl = fmaxf(l - (r + ps), 0.0f);
+            const float lb2 = fmaf(da, da, dl * dl);
+            return lb2 > best2 && best2 < t.disc_limit2 && lb2 < 0x1p17f * t.disc_limit2;
+          };
+          near0 = near0 && !farther(lo2(a), lo2(qq), lo2(czr.y), dslack[0], best[0]);
+          near1 = near1 && !farther(hi2(a), hi2(qq), hi2(czr.y), dslack[1], best[1]);
+        }
+        if (near0 || near1) {  // default.rs:45-49: the minimum of the distances
+          const float4 ra = tl[j].a;
+          const P3 a = p3(ra), b = p3(tl[j].b), c = p3(tl[j].c);
+          const int kind = __float_as_int(ra.w);
+          if (near0) {
+            const float d2 = point_triangle_distance2(p[0], a, b, c, kind);
+            if (d2 < best[0]) {  // fminf: a NaN distance is ignored
+              best[0] = d2;
+              above = pack2(plane_above(d2) + pslack[0], hi2(above));
+            }
+          }
+          if (near1) {
+            const float d2 = point_triangle_distance2(p[1], a, b, c, kind);
+            if (d2 < best[1]) {
+              best[1] = d2;
+              above = pack2(lo2(above), plane_above(d2) + pslack[1]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 0 && i + 2 < ntile) {
+      fence_proxy_async_smem();
+      issue(i + 2);
+    }
+  }
+  if (lost) atomicOr(status, bit(M2S_ERR_LIMIT));
+  for (int u = 0; u < 2; ++u) {
+    if (!valid[u]) continue;
+    if (part) {
+      atomicMin(&part[qi[u]].x, __float_as_uint(best[u]));  // non-negative floats order like their bits
+      if (hits[u] & 1u) atomicXor(&part[qi[u]].y, 1u);
+      continue;
+    }
+    // sqrt(min d2) == min sqrt(d2) (IEEE sqrt is monotone); f32::MAX start value.
+    const float d = fminf(F32_MAX, fsqrt(best[u]));
+    out[qi[u]] = (hits[u] & 1u) ? -d : d;
+  }
+}
+
+// Normal, one thread per query: compare_distances folded over all triangles in
+// order (its ties depend on the order), the reference's fold step for step.
+__global__ void __launch_bounds__(kBfThreads) k_brute_normal(const TriRec* __restrict__ tris, uint32_t T,
+                                                             const float* __restrict__ q, uint64_t nq,
+                                                             float* __restrict__ out, uint32_t* status,
+                                                             const uint32_t* __restrict__ order) {
   __shared__ __align__(128) TriRec tile[2][kBfTile];
-  __shared__ __align__(16) float4 plane_n[2][SIGN == 0 ? kBfTile : 1];  // TriPlane::n
-  __shared__ float plane_s[2][SIGN == 0 ? kBfTile : 1];                  // TriPlane::slack
   __shared__ __align__(8) uint64_t bar[2];
   const int tid = threadIdx.x;
   const uint64_t k = (uint64_t)blockIdx.x * kBfThreads + tid;
   const bool valid = k < nq;
   const uint64_t qi = valid && order ? order[k] : k;  // Morton order: a warp's queries share region branches
   const P3 p = valid ? load_query(q, qi) : P3{0.0f, 0.0f, 0.0f};
-  // this block's chunk of triangles: whole tiles [t_begin, t_end)
-  const uint32_t all_tiles = (T + kBfTile - 1) / kBfTile;
-  const uint32_t per = (all_tiles + gridDim.y - 1) / gridDim.y;
-  const uint32_t t_begin = min(all_tiles, blockIdx.y * per), t_end = min(all_tiles, t_begin + per);
-  const uint32_t ntile = t_end - t_begin;
-  tris += (uint64_t)t_begin * kBfTile;
-  T = ntile == 0 ? 0u : (t_end == all_tiles ? T - t_begin * kBfTile : ntile * kBfTile);
-
+  const uint32_t ntile = (T + kBfTile - 1) / kBfTile;
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
@@ -85,55 +315,22 @@ __global__ void __launch_bounds__(kBfThreads) k_brute(const TriRec* __restrict__
     if (ntile > 0) issue(0);
     if (ntile > 1) issue(1);
   }
-
-  float best = SIGN == 0 ? INFINITY : F32_MAX;  // Raycast keeps the squared distance
-  float reach = INFINITY;                         // Normal: fold_reach(|best|)
-  // Raycast: a triangle's plane bound must exceed `above` to skip it;
-  // `pslack` is the query's share of the bound's slack.
-  float above = INFINITY;
-  const float pslack = plane_query_slack(p);
-  uint32_t hits = 0;
+  float best = F32_MAX, reach = INFINITY;  // reach: fold_reach(|best|)
   bool nan = false, lost = false;
   for (uint32_t i = 0; i < ntile; ++i) {
     const int buf = i & 1;
     if (!mbar_wait_bounded(&bar[buf], (i >> 1) & 1)) lost = true;
     const uint32_t cnt = min((uint32_t)kBfTile, T - i * kBfTile);
     const TriRec* tl = tile[buf];
-    if (SIGN == 0) {
-      lost = __syncthreads_or(lost);  // the planes are only formed from a tile every thread has
-      if (!lost)
-        for (uint32_t j = tid; j < cnt; j += kBfThreads) {
-          const TriPlane pl = tri_plane(p3(tl[j].a), p3(tl[j].b), p3(tl[j].c), __float_as_int(tl[j].a.w));
-          plane_n[buf][j] = pl.n;
-          plane_s[buf][j] = pl.slack;
-        }
-      __syncthreads();
-    }
     if (!lost) {
 #pragma unroll 2
       for (uint32_t j = 0; j < cnt; ++j) {
         const float4 ra = tl[j].a, rb = tl[j].b, rc = tl[j].c;
-        const P3 a = p3(ra), b = p3(rb), c = p3(rc);
-        const int kind = __float_as_int(ra.w);
-        if (SIGN == 0) {
-          // default.rs:45-49 then :59-62 — min of distances, count of +X hits.
-          if (!(plane_bound(plane_n[buf][SIGN == 0 ? j : 0], plane_s[buf][SIGN == 0 ? j : 0], p, pslack) > above)) {
-            const float d2 = point_triangle_distance2(p, a, b, c, kind);
-            if (d2 < best) {  // fminf: a NaN distance is ignored
-              best = d2;
-              above = plane_above(best);
-            }
-          }
-          float t;
-          hits += ray_hit_aligned<0>(p, a, b, c, &t) ? 1u : 0u;
-        } else {
-          // default.rs:51-53 then :63-70 — compare_distances fold; a d
-          // beyond the fold's reach cannot be before best.
-          float d = point_triangle_signed_distance(p, a, b, c, kind);
-          if (!(fabsf(d) > reach) && compare_distances(d, best, &nan) == -1) {
-            best = d;
-            reach = fold_reach(fabsf(best));
-          }
+        // default.rs:51-53 then :63-70; a d beyond the fold's reach cannot be before best.
+        float d = point_triangle_signed_distance(p, p3(ra), p3(rb), p3(rc), __float_as_int(ra.w));
+        if (!(fabsf(d) > reach) && compare_distances(d, best, &nan) == -1) {
+          best = d;
+          reach = fold_reach(fabsf(best));
         }
       }
     }
@@ -145,21 +342,7 @@ __global__ void __launch_bounds__(kBfThreads) k_brute(const TriRec* __restrict__
   }
   if (lost) atomicOr(status, bit(M2S_ERR_LIMIT));
   if (nan) atomicOr(status, bit(M2S_ERR_NAN_DISTANCE));
-  if (!valid) return;
-  if (SIGN == 0 && part) {
-    atomicMin(&part[qi].x, __float_as_uint(best));  // non-negative floats order like their bits
-    if (hits & 1u) atomicXor(&part[qi].y, 1u);
-    return;
-  }
-  float r;
-  if (SIGN == 0) {
-    // sqrt(min d2) == min sqrt(d2) (IEEE sqrt is monotone); f32::MAX start value.
-    float d = fminf(F32_MAX, fsqrt(best));
-    r = (hits & 1u) ? -d : d;
-  } else {
-    r = best;
-  }
-  out[qi] = r;
+  if (valid) out[qi] = best;
 }
 
 __global__ void k_brute_init(uint2* part, uint64_t nq) {
@@ -187,7 +370,7 @@ __global__ void k_brute_finish(const uint2* __restrict__ part, uint64_t nq, floa
 // groups then need no compare_distances at all.
 constexpr int kBwThreads = 256;                 // 8 queries per block
 constexpr uint64_t kBruteWarpMaxQueries = 1u << 17;  // below: one warp per query
-constexpr uint64_t kBruteSortMinPairs = 1ull << 28;  // from here the thread kernels visit queries in Morton order
+constexpr uint64_t kBruteSortMinPairs = 1ull << 24;  // from here the thread kernels visit queries in Morton order
 __global__ void __launch_bounds__(kBwThreads) k_brute_normal_warp(const TriRec* __restrict__ tris, uint32_t T,
                                                                   const float* __restrict__ q, uint64_t nq,
                                                                   float* __restrict__ out, uint32_t* status) {
@@ -291,9 +474,6 @@ __device__ __forceinline__ TriRec load_tri(const TriRec* t, uint32_t i) {
 __device__ __forceinline__ Pill load_pill(const Pill* pills, uint32_t i) {
   const float4* f = reinterpret_cast<const float4*>(pills + i);
   return {__ldg(f), __ldg(f + 1)};
-}
-__device__ __forceinline__ float pill_query_slack(P3 p) {
-  return kPillSlack * fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z)));
 }
 __device__ __forceinline__ float pill_dist2(const Pill& pl, P3 p, float ps) {
   const float x = p.x - pl.a.x, y = p.y - pl.a.y, z = p.z - pl.a.z;
@@ -1334,19 +1514,17 @@ __global__ void k_bf_keys(const float* __restrict__ q, uint64_t nq, const int* _
 int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, float* d_out, uint32_t* d_status,
                     cudaStream_t s, bool allow_alloc) {
   if (nq == 0) return M2S_OK;
-  unsigned blocks = (unsigned)((nq + kBfThreads - 1) / kBfThreads);
-  // Thread-per-query kernels visit large batches (2^28 pairs or more: the
-  // sort's ~20 launches take ~0.1 ms, the order saves ~13 % of the kernel)
-  // in Morton order (of the
-  // queries' own bounding box): the lanes of a warp then mostly fall in the
-  // same Voronoi regions of a triangle and take the same branches (65,536
-  // points x 81,920 triangles Raycast 24.3 -> 21.2 ms, 262,144 Normal 108.5
-  // -> 88.9 ms).  Results are per query, so the order changes none.
+  // Thread-per-query kernels visit batches of 2^24 pairs or more, at least
+  // 1,024 queries, in Morton order (of the queries' own bounding box): the
+  // lanes of a warp then mostly agree on which planes come near and fall in
+  // the same Voronoi regions (Raycast, 10,000 points x 20,480 triangles 0.82
+  // -> 0.52 ms; the sort takes about 0.05 ms).  Results are per query, so the
+  // order changes none.
   DevBuf<uint32_t> keys, order;
   DevBuf<int> bounds;
   const uint32_t* ord = nullptr;
   const bool thread_kernel = sign == M2S_SIGN_RAYCAST || nq >= kBruteWarpMaxQueries;
-  if (allow_alloc && thread_kernel && nq >= 4096 && nq <= 0xFFFFFFFFull && nq * m.n_tris >= kBruteSortMinPairs) {
+  if (allow_alloc && thread_kernel && nq >= 1024 && nq <= 0xFFFFFFFFull && nq * m.n_tris >= kBruteSortMinPairs) {
     int st;
     if ((st = keys.alloc(nq, s)) || (st = order.alloc(nq, s)) || (st = bounds.alloc(6, s))) return st;
     k_bf_bounds_init<<<1, 32, 0, s>>>(bounds.p);
@@ -1358,17 +1536,18 @@ int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, 
   }
   if (sign == M2S_SIGN_RAYCAST) {
     // Enough (query, triangle chunk) blocks to fill the GPU ~4 deep.
-    const uint32_t tiles = (m.n_tris + kBfTile - 1) / kBfTile;
+    const unsigned blocks = (unsigned)((nq + 2 * kBrThreads - 1) / (2 * kBrThreads));
+    const uint32_t tiles = (m.n_tris + kBrTile - 1) / kBrTile;
     uint32_t chunks = (uint32_t)std::max<uint64_t>(1, (148ull * 16ull + blocks - 1) / blocks);
-    chunks = std::max(1u, std::min(chunks, std::min(tiles, 64u)));
+    chunks = std::max(1u, std::min(chunks, std::min(tiles, 256u)));
     if (chunks == 1 || !allow_alloc) {
-      k_brute<0><<<blocks, kBfThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out, d_status, nullptr, ord);
+      k_brute_raycast<<<blocks, kBrThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out, d_status, nullptr, ord);
     } else {
       DevBuf<uint2> part;
       int st = part.alloc(nq, s);
       if (st) return st;
       k_brute_init<<<(unsigned)std::min<uint64_t>((nq + 255) / 256, 148u * 16u), 256, 0, s>>>(part.p, nq);
-      k_brute<0><<<dim3(blocks, chunks), kBfThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out, d_status, part.p, ord);
+      k_brute_raycast<<<dim3(blocks, chunks), kBrThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out, d_status, part.p, ord);
       k_brute_finish<<<(unsigned)std::min<uint64_t>((nq + 255) / 256, 148u * 16u), 256, 0, s>>>(part.p, nq, d_out);
     }
   } else if (nq < kBruteWarpMaxQueries) {
@@ -1379,7 +1558,8 @@ int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, 
     const unsigned wblocks = (unsigned)((nq + kBwThreads / 32 - 1) / (kBwThreads / 32));
     k_brute_normal_warp<<<wblocks, kBwThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out, d_status);
   } else {
-    k_brute<1><<<blocks, kBfThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out, d_status, nullptr, ord);
+    k_brute_normal<<<(unsigned)((nq + kBfThreads - 1) / kBfThreads), kBfThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out,
+                                                                                       d_status, ord);
   }
   M2S_CUDA(cudaGetLastError());
   return M2S_OK;
