@@ -67,6 +67,7 @@ constexpr int kRing = 16;           // buckets of the window
 constexpr int kCur0 = kRing;        // list relaxed first (empty)
 constexpr int kFar0 = kRing + 1;    // far lists kFar0 and kFar0 + 1 (ping-pong)
 constexpr int kLists = kRing + 3;
+constexpr uint32_t kSoloCap = 64;   // largest solo_max
 constexpr uint32_t kNoBucket = 0xFFFFFFFFu;
 constexpr uint32_t kMaxSteps = 1u << 22;  // bound on rounds + redistributions
 constexpr int kAuditStats = 7;
@@ -579,7 +580,7 @@ __device__ __forceinline__ Counters global_counters(PropState* st) { return {st-
 
 __device__ __forceinline__ void push_entry_warp(const Counters& ct, uint32_t b, uint32_t B, const uint32_t* slots,
                                                 uint32_t fp, uint2* lists, uint32_t cap, bool act, uint32_t cell,
-                                                uint32_t tri, uint32_t nb) {
+                                                uint32_t tri, uint32_t nb, uint2* mirror = nullptr) {
   const int lane = threadIdx.x & 31;
   const bool far = act && nb >= B + kRing;
   uint32_t slot = 0xFFFFFFFFu;
@@ -600,6 +601,7 @@ __device__ __forceinline__ void push_entry_warp(const Counters& ct, uint32_t b, 
     lists[(unsigned long long)slot * cap + pos] = make_uint2(cell, tri);
   else
     atomicOr(ct.overflow, 1u);  // the job is rerun with larger lists
+  if (mirror && slot < kFar0 && pos < kSoloCap) mirror[slot * kSoloCap + pos] = make_uint2(cell, tri);
 }
 
 // The same for a whole block at once: the block's states meet in shared
@@ -853,7 +855,6 @@ __device__ __forceinline__ int next_step(Sched& sh, const Counters& ct, uint32_t
 // the waiting blocks' bounded wait always ends.  The work of a round does not
 // depend on which threads do it: results are the same either way.
 constexpr uint32_t kSoloRounds = 1024;  // the threshold (default 64 states) is GridTuning::solo_max
-constexpr uint32_t kSoloCap = 64;  // largest solo_max
 // A run starts at the second small round in a row: an isolated small round
 // (a lull between large ones) costs more as a run of one, which adds a
 // barrier's wait for the other blocks and the schedule handoff, than on every
@@ -862,6 +863,42 @@ constexpr uint32_t kSoloCap = 64;  // largest solo_max
 // 23.7 -> 23.3 ms).  Every block decides from the same schedule.
 __device__ __forceinline__ bool solo_round(const Sched& sh, uint32_t solo_max) {
   return sh.n <= solo_max && sh.prev_n <= solo_max;
+}
+
+// A solo run is the work of block 0's first kSoloThreads threads, which meet
+// at a named barrier of their own.
+constexpr uint32_t kSoloThreads = 512;
+__device__ __forceinline__ void solo_sync(uint32_t threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+
+// What thread 0 of a block notes of its steps, and block 0's log of them.
+struct StepLog {
+  uint32_t* log;  // null: none
+  uint32_t cap, logged, max_list, solo_rounds;
+  uint64_t t0;
+};
+
+// One warp: the next step of schedule `p`.  The leading block's copy is
+// logged when profiling: the relaxed list's size (bit 30: a solo round) or the
+// far list's size (bit 31), and when the step was chosen.
+__device__ __forceinline__ void advance(Sched& p, const Counters& ct, uint32_t spill_overflow, bool leader,
+                                        uint32_t max_steps, uint32_t solo_max, StepLog& lg) {
+  const bool limit = p.steps >= max_steps;
+  const int action = limit ? kLimit : next_step(p, ct, spill_overflow, leader);
+  if ((threadIdx.x & 31u) == 0) {
+    p.action = action;
+    ++p.steps;
+    if (threadIdx.x == 0 && action == kRelax) lg.max_list = max(lg.max_list, p.n);
+    if (leader && lg.log && lg.logged < lg.cap) {
+      uint32_t v = 0;
+      if (action == kRelax) v = p.n | (solo_round(p, solo_max) ? 0x40000000u : 0u);
+      else if (action == kRedistribute) v = 0x80000000u | ct.count[kFar0 + p.fp];
+      else v = 0xC0000000u;  // the end
+      lg.log[2 * lg.logged] = v;
+      lg.log[2 * lg.logged + 1] = (uint32_t)(global_ns() - lg.t0);
+      ++lg.logged;
+    }
+  }
+  __syncwarp();
 }
 
 // Queue of one warp's proposals that need a distance evaluation (Normal sign).
@@ -982,12 +1019,12 @@ __device__ __forceinline__ void table_improve(uint32_t* HJ, unsigned long long* 
 template <int SIGN, bool MULTI>
 __device__ __forceinline__ void relax_propose_solo(const GridSet& gs, const TriRec* __restrict__ tris,
                                                    const unsigned long long* keys, const uint2* list, uint32_t n,
-                                                   uint32_t* HJ, unsigned long long* HK, uint16_t* taken,
-                                                   uint32_t* ntaken, bool& nan, unsigned long long& evals,
-                                                   uint32_t& dropped_same) {
+                                                   uint32_t threads, uint32_t* HJ, unsigned long long* HK,
+                                                   uint16_t* taken, uint32_t* ntaken, bool& nan,
+                                                   unsigned long long& evals, uint32_t& dropped_same) {
   const uint32_t P = 26u * n;
-  for (uint32_t p = threadIdx.x; p < P; p += blockDim.x) {
-    const uint2 ent = __ldcg(&list[p / 26u]);  // written by other blocks in earlier rounds
+  for (uint32_t p = threadIdx.x; p < P; p += threads) {
+    const uint2 ent = list[p / 26u];
     uint32_t j;
     int X, Y, Z;
     if (!neighbour_cell<MULTI>(gs, ent, p % 26u, j, X, Y, Z)) continue;
@@ -1009,11 +1046,12 @@ __device__ __forceinline__ void relax_propose_solo(const GridSet& gs, const TriR
 // Commit phase of a solo round: every taken slot's winner becomes the cell's
 // key and is queued under its bucket; the slot is freed.
 template <bool MULTI>
-__device__ __forceinline__ void relax_commit_solo(const GridSet& gs, unsigned long long* keys, uint32_t* HJ,
-                                                  unsigned long long* HK, const uint16_t* taken, uint32_t ntaken,
-                                                  const Counters& ct, const Sched& sh, uint2* lists, uint32_t cap) {
-  for (uint32_t base = 0; base < ntaken; base += blockDim.x) {  // warp-uniform trip count
-    const uint32_t i = base + threadIdx.x;
+__device__ __forceinline__ void relax_commit_solo(const GridSet& gs, unsigned long long* keys, uint32_t threads,
+                                                  uint32_t* HJ, unsigned long long* HK, const uint16_t* taken,
+                                                  uint32_t ntaken, const Counters& ct, const Sched& sh, uint2* lists,
+                                                  uint32_t cap, uint2* mirror) {
+  for (uint32_t base = threadIdx.x & ~31u; base < ntaken; base += threads) {  // warp-uniform trip count
+    const uint32_t i = base + (threadIdx.x & 31u);
     const bool act = i < ntaken;
     uint32_t j = 0, nb = 0;
     unsigned long long w = KEY_EMPTY;
@@ -1026,7 +1064,92 @@ __device__ __forceinline__ void relax_commit_solo(const GridSet& gs, unsigned lo
       HJ[h] = kNoCell;
       HK[h] = KEY_EMPTY;
     }
-    push_entry_warp(ct, sh.b, sh.B, sh.slot, sh.fp, lists, cap, act, j, key_tri(w), nb);
+    push_entry_warp(ct, sh.b, sh.B, sh.slot, sh.fp, lists, cap, act, j, key_tri(w), nb, mirror);
+  }
+}
+
+// A solo run: block 0 relaxes round after round until one is too large (or the
+// run has lasted kSoloRounds), then leaves the schedule, the next action
+// included, in *sh and st->handoff.
+//
+// Such a round is a chain of dependent steps (the state, its neighbours' keys
+// and triangle, the distance, the table, the pushes, the next list), 5 states
+// wide on average on a 384x384x128 terrain, so what counts is the length of
+// the chain.  The pushes leave a copy of each list's first states in shared
+// memory for the next rounds, every warp advances a copy of the schedule of
+// its own instead of waiting for one that does, and only as many warps take
+// part as shorten a typical round.  Rounds of that terrain's grid (Normal), with
+// the whole block at its own barrier before, now: 3.30 -> 2.3 us up to 7
+// states, 3.65 -> 3.2 up to 15; the grid 17.3 -> 15.7 ms (128 / 256 / 512 /
+// 1,024 threads of the run: 16.8 / 15.9 / 15.7 / 16.2).  The schedule's state
+// leaves the other rounds' registers, which then do not spill for Raycast:
+// 256^3 8.35 -> 8.02 ms, 24 grids of 32M cells 21.5 -> 20.6.  Out of line the
+// run costs the terrain 16.1 ms.
+template <int SIGN, bool MULTI>
+__device__ __forceinline__ void solo_run(const GridSet& gs, const TriRec* __restrict__ tris,
+                                         unsigned long long* keys, uint2* lists, uint32_t cap, PropState* st,
+                                         Sched* sh, StepLog* lg, uint32_t max_steps, uint32_t solo_max, bool& nan,
+                                         unsigned long long& evals, uint32_t& dropped_same) {
+  extern __shared__ __align__(16) uint32_t s_touch[];
+  __shared__ uint16_t s_taken[26 * kSoloCap];       // a round's taken table slots
+  __shared__ uint32_t s_ntaken[2];
+  __shared__ uint32_t s_count[kLists], s_far_min[2], s_overflow;  // the counters: block 0 alone pushes
+  __shared__ Sched s_plan[kSoloThreads / 32];       // the schedule, a copy for each warp
+  __shared__ uint2 s_mirror[kFar0 * kSoloCap];      // each list's first states
+  uint32_t* HJ = s_touch;  // the min table, kept empty between rounds
+  unsigned long long* HK = reinterpret_cast<unsigned long long*>(s_touch + kHash);
+  const uint32_t threads = min(blockDim.x, kSoloThreads);
+  if (threadIdx.x < kLists) s_count[threadIdx.x] = *(volatile uint32_t*)&st->count[threadIdx.x];
+  if (threadIdx.x == 32) {
+    s_far_min[0] = *(volatile uint32_t*)&st->far_min[0];
+    s_far_min[1] = *(volatile uint32_t*)&st->far_min[1];
+    s_overflow = *(volatile uint32_t*)&st->overflow | *(volatile uint32_t*)&st->overflow2[0] |
+                 *(volatile uint32_t*)&st->overflow2[1];
+    s_ntaken[0] = s_ntaken[1] = 0;
+  }
+  for (uint32_t h = threadIdx.x; h < kHash; h += blockDim.x) {
+    HJ[h] = kNoCell;
+    HK[h] = KEY_EMPTY;
+  }
+  for (uint32_t i = threadIdx.x; i < kFar0 * kSoloCap; i += blockDim.x) {
+    const uint32_t k = i / kSoloCap, e = i % kSoloCap;
+    if (e < min(*(volatile uint32_t*)&st->count[k], cap))
+      s_mirror[i] = __ldcg(&lists[(unsigned long long)k * cap + e]);
+  }
+  if (threadIdx.x < threads && (threadIdx.x & 31u) == 0) s_plan[threadIdx.x >> 5] = *sh;
+  __syncthreads();
+  if (threadIdx.x < threads) {
+    Sched& plan = s_plan[threadIdx.x >> 5];
+    const Counters ct{s_count, s_far_min, &s_overflow};
+    unsigned long long entries = 0;
+    uint32_t runs = 0;
+    bool more;
+    do {
+      const uint32_t turn = runs & 1u;
+      entries += plan.n;
+      relax_propose_solo<SIGN, MULTI>(gs, tris, keys, s_mirror + plan.cur * kSoloCap, min(plan.n, cap), threads, HJ,
+                                      HK, s_taken, &s_ntaken[turn], nan, evals, dropped_same);
+      solo_sync(threads);
+      if (threadIdx.x == 0) s_ntaken[turn ^ 1u] = 0;  // read in the round before
+      relax_commit_solo<MULTI>(gs, keys, threads, HJ, HK, s_taken, min(s_ntaken[turn], 26u * kSoloCap), ct, plan,
+                               lists, cap, s_mirror);
+      solo_sync(threads);
+      advance(plan, ct, 0u, threadIdx.x < 32, max_steps, solo_max, *lg);
+      ++runs;
+      more = plan.action == kRelax && solo_round(plan, solo_max) && runs < kSoloRounds;
+    } while (more);
+    if (threadIdx.x == 0) {
+      lg->solo_rounds += runs;
+      atomicAdd(&st->entries, entries);
+      for (int k = 0; k < kLists; ++k) st->count[k] = s_count[k];
+      st->far_min[0] = s_far_min[0];
+      st->far_min[1] = s_far_min[1];
+      if (s_overflow) st->overflow = 1u;
+      *sh = plan;
+      volatile uint32_t* dst = (volatile uint32_t*)&st->handoff;
+      const uint32_t* src = (const uint32_t*)&plan;
+      for (uint32_t w = 0; w < sizeof(Sched) / 4; ++w) dst[w] = src[w];
+    }
   }
 }
 
@@ -1358,15 +1481,10 @@ __global__ void __launch_bounds__(FILTER ? kSmallBlock : kBigBlock, FILTER ? 3 :
   __shared__ Sched sh;
   // [cells touched this round (also a solo run's min table) | the warps' queues]
   extern __shared__ __align__(16) uint32_t s_touch[];
-  __shared__ uint16_t s_taken[26 * kSoloCap];              // a solo round's taken table slots
   constexpr bool kQueued = SIGN == M2S_SIGN_NORMAL || FILTER;  // the plain Raycast loop needs no queue
   WarpQueue* s_queue = reinterpret_cast<WarpQueue*>(s_touch + kStagePerThread * blockDim.x);
-  __shared__ uint32_t s_ntouch, s_gen, s_pending, s_more, s_runs, s_solo_run;
-  __shared__ uint32_t s_count[kLists], s_far_min[2], s_overflow;  // block 0's counters during a solo run
-  // (built where used, so no pointer stays live across the propose loop)
-  auto counters = [&](bool shared_ones) {
-    return shared_ones ? Counters{s_count, s_far_min, &s_overflow} : global_counters(st);
-  };
+  __shared__ uint32_t s_ntouch, s_gen, s_pending;
+  __shared__ StepLog s_log;
   const unsigned int nblocks = gridDim.x;
   const int lane = threadIdx.x & 31;
   const bool lead_block = blockIdx.x == 0;
@@ -1374,8 +1492,6 @@ __global__ void __launch_bounds__(FILTER ? kSmallBlock : kBigBlock, FILTER ? 3 :
     s_ntouch = 0;
     s_gen = 0;
     s_pending = 0;
-    s_runs = 0;
-    s_solo_run = 0;
     sh.b = st->b;
     sh.B = st->B;
     for (int k = 0; k < kRing; ++k) sh.slot[k] = st->slot[k];
@@ -1384,6 +1500,7 @@ __global__ void __launch_bounds__(FILTER ? kSmallBlock : kBigBlock, FILTER ? 3 :
     sh.round = 0;
     sh.steps = 0;
     sh.n = 0xFFFFFFFFu;  // no relax round yet: the first is never solo
+    s_log = {lead_block ? round_log : nullptr, log_cap, 0, 0, 0, lead_block && round_log ? global_ns() : 0};
   }
   __shared__ BlockPush s_push;
   block_push_init(&s_push);  // the first step's barrier follows
@@ -1391,49 +1508,22 @@ __global__ void __launch_bounds__(FILTER ? kSmallBlock : kBigBlock, FILTER ? 3 :
   bool nan = false;
   unsigned long long evals = 0;
   uint32_t dropped_same = 0, dropped_bound = 0;
-  uint32_t far_phases = 0, logged = 0, max_list = 0, solo_rounds = 0;
-  const uint64_t t_start = (lead_block && threadIdx.x == 0 && round_log) ? global_ns() : 0;
+  uint32_t far_phases = 0;
   bool aborted = false;
-  // Warp 0: the next step (unless a solo run already chose it), logged by
-  // block 0 when profiling: the relaxed list's size, or (top bit) the far list's.
-  auto step = [&]() {
-    const bool in_run = lead_block && s_solo_run;
-    const uint32_t spill_ov = in_run ? 0u : *(volatile uint32_t*)&st->overflow2[sh.round & 1u];
-    const bool limit = sh.steps >= max_steps;
-    const int action = limit ? kLimit : next_step(sh, counters(in_run), spill_ov, lead_block);
-    if (threadIdx.x != 0) {
-      __syncwarp();
-      return;
-    }
-    s_ntouch = 0;  // every thread read it in the last commit, before the last barrier
-    sh.action = action;
-    ++sh.steps;
-    if (sh.action == kRelax) max_list = max(max_list, sh.n);
-    // Profiling: block 0 records each step — the relaxed list's size (bit 30:
-    // a solo round) or the far list's size (bit 31) — and when it was chosen.
-    if (lead_block && round_log && logged < log_cap) {
-      uint32_t v = 0;
-      if (sh.action == kRelax) v = sh.n | (solo_round(sh, solo_max) ? 0x40000000u : 0u);
-      else if (sh.action == kRedistribute) v = 0x80000000u | counters(in_run).count[kFar0 + sh.fp];
-      else v = 0xC0000000u;  // the end
-      round_log[2 * logged] = v;
-      round_log[2 * logged + 1] = (uint32_t)(global_ns() - t_start);
-      ++logged;
-    }
-    __syncwarp();
-  };
-  bool chosen = false;  // a solo round's tail chose this step already (block-uniform)
   for (;;) {
-    if (!chosen) {
-      if (threadIdx.x < 32) {
-        const bool pending = s_pending;
-        __syncwarp();
-        if (!pending) step();
-        else if (threadIdx.x == 0) s_pending = 0;
+    if (threadIdx.x < 32) {
+      const bool pending = s_pending;  // a solo run left the next step chosen
+      __syncwarp();
+      if (!pending) {
+        if (threadIdx.x == 0) s_ntouch = 0;  // every thread read it in the last commit, before the last barrier
+        advance(sh, global_counters(st), *(volatile uint32_t*)&st->overflow2[sh.round & 1u], lead_block, max_steps,
+                solo_max, s_log);
+      } else if (threadIdx.x == 0) {
+        s_pending = 0;
+        s_ntouch = 0;
       }
-      __syncthreads();
     }
-    chosen = false;
+    __syncthreads();
     const int action = sh.action;
     if (action == kDone) break;
     if (action == kLimit) {
@@ -1487,109 +1577,49 @@ __global__ void __launch_bounds__(FILTER ? kSmallBlock : kBigBlock, FILTER ? 3 :
       continue;
     }
     // ---- a relax round: by every block, or by block 0 alone when it is small
-    const bool solo = solo_round(sh, solo_max);
-    if (solo && !s_solo_run) {
-      // A solo run starts.  Block 0 will change list counts at once (pushes,
-      // and emptying the list it relaxes at its next step), so every block
-      // first finishes reading this step's counts.
+    if (solo_round(sh, solo_max)) {
+      // A solo run.  Block 0 will change list counts at once (pushes, and
+      // emptying the list it relaxes at its next step), so every block first
+      // finishes reading this step's counts.
       if (!grid_barrier(bar, nblocks, &s_gen)) {
         aborted = true;
         break;
       }
-      if (!lead_block) {  // wait for the run to end, then take block 0's schedule
-        if (!grid_barrier(bar, nblocks, &s_gen)) {
-          aborted = true;
-          break;
-        }
-        if (threadIdx.x == 0) {
-          const volatile uint32_t* src = (const volatile uint32_t*)&st->handoff;
-          uint32_t* dst = (uint32_t*)&sh;
-          for (uint32_t w = 0; w < sizeof(Sched) / 4; ++w) dst[w] = src[w];
-          s_pending = 1;
-        }
-        continue;
+      if (lead_block) {
+        solo_run<SIGN, MULTI>(gs, tris, keys, lists, cap, st, &sh, &s_log, max_steps, solo_max, nan,
+                              evals, dropped_same);
+        if (threadIdx.x == 0) s_pending = 1;
       }
-      if (threadIdx.x == 0) {
-        // Block 0 alone pushes during the run: it keeps the counters in shared
-        // memory and writes them back when it hands the schedule over.
-        s_solo_run = 1;  // read again only after later block barriers
-        for (int k = 0; k < kLists; ++k) s_count[k] = *(volatile uint32_t*)&st->count[k];
-        s_far_min[0] = *(volatile uint32_t*)&st->far_min[0];
-        s_far_min[1] = *(volatile uint32_t*)&st->far_min[1];
-        s_overflow = *(volatile uint32_t*)&st->overflow | *(volatile uint32_t*)&st->overflow2[0] |
-                     *(volatile uint32_t*)&st->overflow2[1];
+      // The other blocks wait for the run to end, then take block 0's schedule.
+      if (!grid_barrier(bar, nblocks, &s_gen)) {
+        aborted = true;
+        break;
       }
-      for (uint32_t h = threadIdx.x; h < kHash; h += blockDim.x) {  // the run's min table, kept empty between rounds
-        s_touch[h] = kNoCell;
-        reinterpret_cast<unsigned long long*>(s_touch + kHash)[h] = KEY_EMPTY;
+      if (!lead_block && threadIdx.x == 0) {
+        const volatile uint32_t* src = (const volatile uint32_t*)&st->handoff;
+        uint32_t* dst = (uint32_t*)&sh;
+        for (uint32_t w = 0; w < sizeof(Sched) / 4; ++w) dst[w] = src[w];
+        s_pending = 1;
       }
-      __syncthreads();
+      continue;
     }
     const uint32_t parity = sh.round & 1u;
     uint32_t* spill = spill_lists + (unsigned long long)parity * cap;
     const uint32_t n = min(sh.n, cap);
-    const uint32_t T = solo ? blockDim.x : gridDim.x * blockDim.x;
-    const uint32_t t0 = solo ? threadIdx.x : blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t* HJ = s_touch;
-    unsigned long long* HK = reinterpret_cast<unsigned long long*>(s_touch + kHash);
-    if (solo)
-      relax_propose_solo<SIGN, MULTI>(gs, tris, keys, lists + (unsigned long long)sh.cur * cap, n, HJ, HK,
-                                      s_taken, &s_ntouch, nan, evals, dropped_same);
-    else
-      relax_propose<SIGN, MULTI, FILTER>(gs, tris, bounds, slack, keys,
-                                 lists + (unsigned long long)sh.cur * cap, n, T, t0, s_touch, &s_ntouch, st, parity,
-                                 spill, cap, nan, evals, dropped_same, dropped_bound,
-                                         &s_queue[kQueued ? threadIdx.x >> 5 : 0]);
+    const uint32_t T = gridDim.x * blockDim.x;
+    const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    relax_propose<SIGN, MULTI, FILTER>(gs, tris, bounds, slack, keys, lists + (unsigned long long)sh.cur * cap, n, T,
+                                       t0, s_touch, &s_ntouch, st, parity, spill, cap, nan, evals, dropped_same,
+                                       dropped_bound, &s_queue[kQueued ? threadIdx.x >> 5 : 0]);
     if (lead_block && threadIdx.x == 0) atomicAdd(&st->entries, (unsigned long long)n);
-    if (solo) {
-      __syncthreads();
-    } else if (!grid_barrier(bar, nblocks, &s_gen)) {
+    if (!grid_barrier(bar, nblocks, &s_gen)) {
       aborted = true;
       break;
     }
-    if (solo) {
-      relax_commit_solo<MULTI>(gs, keys, HJ, HK, s_taken, min(s_ntouch, 26u * kSoloCap),
-                               counters(true), sh, lists, cap);
-    } else {
-      if (lead_block && threadIdx.x == 0) st->touched2[parity ^ 1u] = 0;
-      const uint32_t nspill = min(*(volatile uint32_t*)&st->touched2[parity], cap);
-      relax_commit<MULTI>(gs, keys, s_touch, min(s_ntouch, kStagePerThread * blockDim.x), spill, nspill, t0,
-                          T, st, sh, lists, cap, &s_push, push_turn);
-    }
-    if (!solo) {
-      if (!grid_barrier(bar, nblocks, &s_gen)) {
-        aborted = true;
-        break;
-      }
-      continue;
-    }
-    // Solo: block 0 chooses the next step at once; it goes on alone while the
-    // rounds stay small, else hands the schedule (next action included) to the
-    // other blocks at the barrier they wait at.
-    __syncthreads();
-    if (threadIdx.x < 32) step();
-    if (threadIdx.x == 0) {
-      ++s_runs;
-      ++solo_rounds;
-      s_more = sh.action == kRelax && solo_round(sh, solo_max) && s_runs < kSoloRounds;
-      if (!s_more) {
-        for (int k = 0; k < kLists; ++k) st->count[k] = s_count[k];
-        st->far_min[0] = s_far_min[0];
-        st->far_min[1] = s_far_min[1];
-        if (s_overflow) st->overflow = 1u;
-        volatile uint32_t* dst = (volatile uint32_t*)&st->handoff;
-        const uint32_t* src = (const uint32_t*)&sh;
-        for (uint32_t w = 0; w < sizeof(Sched) / 4; ++w) dst[w] = src[w];
-        s_runs = 0;
-        s_solo_run = 0;
-        s_pending = 1;
-      }
-    }
-    __syncthreads();
-    if (s_more) {
-      chosen = true;
-      continue;
-    }
+    if (lead_block && threadIdx.x == 0) st->touched2[parity ^ 1u] = 0;
+    const uint32_t nspill = min(*(volatile uint32_t*)&st->touched2[parity], cap);
+    relax_commit<MULTI>(gs, keys, s_touch, min(s_ntouch, kStagePerThread * blockDim.x), spill, nspill, t0, T, st, sh,
+                        lists, cap, &s_push, push_turn);
     if (!grid_barrier(bar, nblocks, &s_gen)) {
       aborted = true;
       break;
@@ -1609,9 +1639,9 @@ __global__ void __launch_bounds__(FILTER ? kSmallBlock : kBigBlock, FILTER ? 3 :
   if (lead_block && threadIdx.x == 0) {
     st->round = sh.round;
     st->far_phases = far_phases;
-    st->log_n = logged;
-    st->max_list = max_list;
-    st->solo_rounds = solo_rounds;
+    st->log_n = s_log.logged;
+    st->max_list = s_log.max_list;
+    st->solo_rounds = s_log.solo_rounds;
     st->done = 1;
   }
 }
