@@ -774,14 +774,14 @@ __device__ bool nearest_triangle_warp(const MeshView& m, P3 p, Nearest* io, uint
     if (node != 0xFFFFFFFFu && nd2 <= bound) {
       if constexpr (STATS) ++qc->visits;
       BvhNode nd = load_node(m.nodes, node);
-      // (with the node: a step's time is its chain of dependent loads)
-      const Pill pl[2] = {load_pill(m.pills, 2u * node), load_pill(m.pills, 2u * node + 1u)};
-      const float limit[2] = {nd.r_lo.w, nd.r_hi.w};
       const uint32_t ch[2] = {__float_as_uint(nd.l_lo.w), __float_as_uint(nd.l_hi.w)};
       float cd[2] = {box_dist2(p, nd.l_lo, nd.l_hi), box_dist2(p, nd.r_lo, nd.r_hi)};
+      // (fetched only where they may prune: with every node they were 64 bytes a
+      // child pair that a rough mesh seldom uses, terrain 512^2 Bvh(Normal)
+      // 60,000 points 1.35 -> 1.18 ms, Rtree 100,000 1.06 -> 1.01, stars even)
+      pill_raise(m.pills, node, nd.r_lo.w, nd.r_hi.w, p, ps, bound, &cd[0], &cd[1]);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        if (cd[c] <= bound && bound < limit[c]) cd[c] = fmaxf(cd[c], pill_dist2(pl[c], p, ps));
         if (!(cd[c] <= bound)) continue;
         if (ch[c] & LEAF_BIT) {
           const uint32_t leaf = ch[c] & ~LEAF_BIT;
@@ -1161,13 +1161,11 @@ __device__ bool normal_band_fold_warp(const MeshView& m, P3 p, float d2min, uint
       if (node != 0xFFFFFFFFu) {
         if constexpr (STATS) ++qc->sign_visits;
         const BvhNode nd = load_node(m.nodes, node);
-        const Pill pl[2] = {load_pill(m.pills, 2u * node), load_pill(m.pills, 2u * node + 1u)};
-        const float limit[2] = {nd.r_lo.w, nd.r_hi.w};
         const uint32_t ch[2] = {__float_as_uint(nd.l_lo.w), __float_as_uint(nd.l_hi.w)};
         float cd[2] = {box_dist2(p, nd.l_lo, nd.l_hi), box_dist2(p, nd.r_lo, nd.r_hi)};
+        pill_raise(m.pills, node, nd.r_lo.w, nd.r_hi.w, p, ps, reach2, &cd[0], &cd[1]);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-          if (cd[c] <= reach2 && reach2 < limit[c]) cd[c] = fmaxf(cd[c], pill_dist2(pl[c], p, ps));
           if (!(cd[c] <= reach2)) continue;
           if (ch[c] & LEAF_BIT) consider(ch[c] & ~LEAF_BIT);
           else push[npush++] = ch[c];
