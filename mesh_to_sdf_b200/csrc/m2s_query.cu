@@ -1459,15 +1459,29 @@ __global__ void k_query_keys(const float* __restrict__ q, uint64_t nq, MeshView 
 // Node-visit budget of the single-thread search (0: single pass only).
 std::atomic<uint32_t> g_query_budget{768};
 
-// Batches up to this many queries run one warp per query (k_query_warpwise), on
-// meshes of up to kWarpwiseSmallMesh triangles and on larger ones, whose
-// searches fill the warp's lanes for longer.  Measured on B200 against the
-// two-pass path: 10,000 queries on star s3 (1,280 triangles) 0.12 against 0.15
-// ms, s5 (20,480) 0.22 / 0.22; s6 (81,920) 4,000 queries 0.19 against 0.23 ms,
-// 6,000 0.26 / 0.25, the terrain strip (524,282) 0.14 / 0.15 and 0.21 / 0.16
-// (bit-identical throughout).
-constexpr uint64_t kWarpwiseMaxQueries = 10240, kWarpwiseMaxLarge = 4096;
-constexpr uint32_t kWarpwiseSmallMesh = 1u << 15;
+// Batches up to this many queries run one warp per query (k_query_warpwise).
+// The line is where one thread per query (with its warp pass) gets ahead.
+// Methods that vote with three rays reach it latest (a thread casts its rays
+// one after another, a warp 32 nodes at a time), Bvh(Normal) with its band
+// fold later than Rtree.  Measured on B200, a warp per query / the two-pass
+// path in us, bit-identical throughout, on the terrain of 44,994, 145,794 and
+// 524,282 triangles and the star of 81,920:
+//   RtreeBvh     8,192: 161 / 350   193 / 467   258 / 686   267 / 261
+//   Bvh(Normal)  5,000: 116 / 154   135 / 176   183 / 206   176 / 164
+//                8,192: 175 / 188   212 / 206   285 / 249   264 / 207
+//   Rtree        5,000:  83 / 103   103 / 113   149 / 143   151 / 119
+//                7,000: 110 / 122   140 / 139   204 / 168   195 / 136
+// and at 10,240 on terrains of up to 31,746 RtreeBvh 169 / 339, Rtree 127 / 130,
+// on the star's 20,480 236 / 227 and 187 / 125 (5,120: 161 / 188, 118 / 108).
+// With 4,096 as the line of every mesh above 2^15 the terrains' RtreeBvh
+// batches up to 8,192 ran at 0.33 to 0.43 times the speed.
+inline uint64_t warpwise_max(int mode, uint32_t n_tris) {
+  if (n_tris <= 1u << 15) return 10240;
+  const bool large = n_tris > 1u << 16;
+  if (mode == Q_RTREE) return large ? 4096 : 6144;
+  if (mode == Q_BVH_NORMAL) return large ? 5120 : 8192;
+  return 8192;
+}
 constexpr uint64_t kMortonMinQueries = 1u << 17;  // batch size from which queries run in Morton order
 
 namespace {
@@ -1620,7 +1634,7 @@ int query_points(const MeshView& m, int accel, int sign, const float* d_q, uint6
                                 ? Q_RTREE
                                 : ((accel == M2S_ACCEL_BVH && sign == M2S_SIGN_NORMAL) ? Q_BVH_NORMAL : Q_BVH_RAYCAST));
   // Small batches (a mesh of more than one triangle): one warp per query.
-  if (nq <= (m.n_tris <= kWarpwiseSmallMesh ? kWarpwiseMaxQueries : kWarpwiseMaxLarge) && !(m.root & LEAF_BIT)) {
+  if (nq <= warpwise_max(mode, m.n_tris) && !(m.root & LEAF_BIT)) {
     const bool counting = profiling_enabled() || grid_tuning().fp64_audit;
     DevBuf<unsigned long long> qs;
     int st;
