@@ -13,6 +13,7 @@
 
 #include "../../include/m2s.h"
 #include "m2s_geo.cuh"
+#include "m2s_reach.cuh"
 
 namespace m2s {
 
@@ -53,17 +54,11 @@ struct __align__(16) Pill {
 // Children of more leaves than this have no pillbox (a large patch is not
 // flat, and building it would read every leaf once per level).
 constexpr uint32_t kPillLeaves = 256;
-// A pillbox prunes a search whose best distance is at most this many times
-// the smallest Q of its triangles, Q = (twice the area) * (shortest edge) /
-// (longest edge)^2.  The reference's f32 closest point (closest_point_proper)
-// can leave a triangle only in the face region, when rounding hides that the
-// foot of the perpendicular lies outside an edge line: by at most
-// o = 24 u D^2 / Q at distance D (u = 2^-24: each of the products d1 d4 - d3 d2
-// errs by 24 u (longest edge)^2 D^2), which brings the point nearer than the
-// triangle by o^2 / (2 D).  At D = 1024 Q that is below 20 u D, well inside
-// the slack of 2^-17 = 128 u of the coordinates' magnitudes.  In every other
-// region the point lies on the triangle up to rounding.
-constexpr float kPillReach = 1024.0f;
+// A pillbox prunes a search whose best distance is at most the least reach of
+// its triangles (m2s_reach.cuh), where the reference's own f32 distance is
+// proven to lie above the bound.  The box test before it puts the query within
+// that distance of the child's box, so a box of at most kReachSpan reaches keeps
+// every triangle of the child within the distances the proof covers.
 // Slack of a pillbox per unit of coordinate magnitude: the node's share is in
 // h and r, the query's is added by the search.
 constexpr float kPillSlack = 0x1p-17f;

@@ -227,7 +227,7 @@ __device__ __forceinline__ Pill make_pill(const TriRec* __restrict__ stris, uint
     return P3{uy * vz - uz * vy, uz * vx - ux * vz, ux * vy - uy * vx};
   };
   const P3 ref = area(stris[first]);
-  float nx = 0.f, ny = 0.f, nz = 0.f, limit = INFINITY;
+  float nx = 0.f, ny = 0.f, nz = 0.f, limit = INFINITY;  // limit: the least reach
   float lox = INFINITY, loy = INFINITY, loz = INFINITY, hix = -INFINITY, hiy = -INFINITY, hiz = -INFINITY;
   for (uint32_t k = first + lane; k <= last; k += LANES) {
     const TriRec t = stris[k];
@@ -242,17 +242,7 @@ __device__ __forceinline__ Pill make_pill(const TriRec* __restrict__ stris, uint
     hix = fmaxf(hix, fmaxf(t.a.x, fmaxf(t.b.x, t.c.x)));
     hiy = fmaxf(hiy, fmaxf(t.a.y, fmaxf(t.b.y, t.c.y)));
     hiz = fmaxf(hiz, fmaxf(t.a.z, fmaxf(t.b.z, t.c.z)));
-    if (__float_as_int(t.a.w) == TRI_PROPER) {
-      auto len2 = [](float4 p, float4 q) {
-        const float x = p.x - q.x, y = p.y - q.y, z = p.z - q.z;
-        return x * x + y * y + z * z;
-      };
-      const float e0 = len2(t.a, t.b), e1 = len2(t.b, t.c), e2 = len2(t.c, t.a);
-      const float q = sqrtf(w.x * w.x + w.y * w.y + w.z * w.z) * sqrtf(fminf(e0, fminf(e1, e2))) /
-                      fmaxf(e0, fmaxf(e1, e2));
-      limit = q > 0.f ? fminf(limit, q) : 0.f;  // also 0 where the area underflows or anything is NaN
-      if (!(q > 0.f)) limit = 0.f;
-    }
+    if (__float_as_int(t.a.w) == TRI_PROPER) limit = fminf(limit, tri_reach(&t.a.x, &t.b.x, &t.c.x));
   }
   nx = sum(nx);
   ny = sum(ny);
@@ -304,15 +294,17 @@ __device__ __forceinline__ Pill make_pill(const TriRec* __restrict__ stris, uint
   const float slack = kPillSlack * scale;
   auto up16 = [](float v) { return (__float_as_uint(v) + 0xFFFFu) >> 16; };  // v >= 0
   const float hs = h + slack, rs = sqrtf(r2) * 1.00001f + slack;
-  const float reach = kPillReach * limit;
-  // NaN or infinite vertices, and magnitudes whose squares overflow: never prune.
-  const bool fine = hs < 0x1p60f && rs < 0x1p60f && scale < 0x1p60f;
+  const float bx = hix - lox + 2e-4f, by = hiy - loy + 2e-4f, bz = hiz - loz + 2e-4f;  // the padded box
+  const float limit2 = fminf(limit * limit, 0x1p126f);
+  // NaN, infinite or huge vertices, and boxes of many reaches: never prune.
+  const bool fine = hs < 0x1p60f && rs < 0x1p60f && scale < kReachScale &&
+                    bx * bx + by * by + bz * bz <= kReachSpan * kReachSpan * limit2;
   // Where the pillbox is not much flatter than the box is along its axis, the
   // box alone prunes about as well: a search then skips it (limit 0).
   const float flat = 0.5f * ((hix - lox) * fabsf(nx) + (hiy - loy) * fabsf(ny) + (hiz - loz) * fabsf(nz));
   Pill p;
   p.a = make_float4(cx, cy, cz, __uint_as_float(fine ? (up16(hs) << 16) | up16(rs) : 0u));
-  p.b = make_float4(nx, ny, nz, fine && h < kPillFlat * flat ? fminf(reach * reach, 0x1p126f) : 0.0f);
+  p.b = make_float4(nx, ny, nz, fine && h < kPillFlat * flat ? limit2 : 0.0f);
   return p;
 }
 

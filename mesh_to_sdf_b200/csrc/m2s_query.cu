@@ -56,10 +56,9 @@ constexpr int kBfTile = 256;  // triangles per stage: 256 * 48 B = 12 KiB
 // the plane comes near (a third of the planes of a closed mesh, for a point
 // outside it), the disc around the triangle decides in the same way: the bound
 // of Pill (m2s_internal.cuh) with a single triangle, for triangles whose angle
-// at a has sin^2 >= 1/200 as for the plane.  Below the reach the reference's
-// point leaves the disc by less than the slack, and at up to 2^8.5 times the
-// reach it errs by less than a fifth of the distance, so the triangle is still
-// the farther one; beyond that the disc says nothing.
+// at a has sin^2 >= 1/200 as for the plane, while the best distance is within
+// the triangle's reach and the bound below 2^8.5 reaches (m2s_reach.cuh covers
+// 370, and the disc itself is less than 6 reaches wide).
 // Rust's f32::min ignores a NaN distance (default.rs:58), so a skipped
 // triangle changes nothing even then.
 //
@@ -192,13 +191,10 @@ __global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* _
         return (u.x - x) * (u.x - x) + (u.y - y) * (u.y - y) + (u.z - z) * (u.z - z);
       };
       const float r2 = fmaxf(len2(t0, cx, cy, cz), fmaxf(len2(t1, cx, cy, cz), len2(t2, cx, cy, cz)));
-      const float e0 = len2(t0, t1.x, t1.y, t1.z), e1 = len2(t1, t2.x, t2.y, t2.z), e2 = len2(t2, t0.x, t0.y, t0.z);
-      const P3 w = vcross(vsub(t1, t0), vsub(t2, t0));
-      const float reach = kPillReach * sqrtf(w.x * w.x + w.y * w.y + w.z * w.z) * sqrtf(fminf(e0, fminf(e1, e2))) /
-                          fmaxf(e0, fmaxf(e1, e2));
       const float slack = pl.slack * (kPillSlack / 0x1p-11f);  // the plane's is 2^-11 of the magnitude
       pair[tid].disc_slack = slack;
-      pair[tid].disc_limit2 = pl.slack < INFINITY && reach > 0.0f ? fminf(reach * reach, 0x1p100f) : 0.0f;
+      const float reach = pl.slack < kReachScale * 0x1p-11f ? tri_reach(&tl[tid].a.x, &tl[tid].b.x, &tl[tid].c.x) : 0.0f;
+      pair[tid].disc_limit2 = reach * reach;
       const float r = sqrtf(r2) * 1.00001f + slack;
       pair[tid].cxy = twice(-cx, -cy);
       pair[tid].czr = twice(-cz, r);
