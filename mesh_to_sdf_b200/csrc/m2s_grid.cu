@@ -445,22 +445,24 @@ __global__ void k_init(ulonglong2* keys2, unsigned long long ncell, PropState* s
 // coarse mesh in a fine grid; the long windows that join a strip's rows) would
 // keep its warp busy long after the others have left (the terrain strip's
 // seeding: 1.62 ms, 0.60 + 0.12 ms with the split), so a box of more than kSplitCells cells is left in
-// chunks of kChunkCells for a second kernel, a warp each.  The list holds
-// kMaxChunks; a triangle that does not fit stays with its warp.
+// chunks of kChunkCells for a second kernel, a warp each.  The list lies in the
+// memory of the bucket lists, which hold nothing yet when seeding runs and
+// nothing any more when the rays do; it takes kMaxChunks of it at most, and a
+// triangle that does not fit stays with its warp.
 constexpr uint32_t kSplitCells = 1024, kChunkCells = 512, kMaxChunks = 1u << 18;
 constexpr uint32_t kNoChunk = 0xFFFFFFFFu;
 // Lists the chunks of triangle t (each as (t, first + chunk * step)) and
 // returns true, or returns false: the caller does the whole box.  All 32 lanes call it.
 __device__ __forceinline__ bool split_box(uint32_t t, unsigned long long total, uint32_t first, uint32_t step,
-                                          uint32_t* count, uint2* chunks) {
-  if (total <= kSplitCells || total > (unsigned long long)kMaxChunks * kChunkCells) return false;
+                                          uint32_t* count, uint2* chunks, uint32_t max_chunks) {
+  if (total <= kSplitCells || total > (unsigned long long)max_chunks * kChunkCells) return false;
   const uint32_t lane = threadIdx.x & 31u, nch = (uint32_t)((total + kChunkCells - 1) / kChunkCells);
   // (Once the list is full nobody adds: the counter cannot wrap.)
-  uint32_t base = kMaxChunks;
-  if (lane == 0 && *(volatile uint32_t*)count < kMaxChunks) base = atomicAdd(count, nch);
+  uint32_t base = max_chunks;
+  if (lane == 0 && *(volatile uint32_t*)count < max_chunks) base = atomicAdd(count, nch);
   base = __shfl_sync(0xFFFFFFFFu, base, 0);
-  const bool fits = base < kMaxChunks && nch <= kMaxChunks - base;
-  for (uint32_t k = lane; k < nch && base < kMaxChunks && base + k < kMaxChunks; k += 32u)
+  const bool fits = base < max_chunks && nch <= max_chunks - base;
+  for (uint32_t k = lane; k < nch && base < max_chunks && base + k < max_chunks; k += 32u)
     chunks[base + k] = make_uint2(fits ? t : kNoChunk, first + k * step);
   return fits;
 }
@@ -516,7 +518,7 @@ __device__ __forceinline__ void seed_cells(const GridK& g, const TriRec& r, uint
 
 template <int SIGN, bool MULTI>
 __global__ void k_seed(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t T,
-                       unsigned long long* keys, uint32_t* status, PropState* st, uint2* chunks) {
+                       unsigned long long* keys, uint32_t* status, PropState* st, uint2* chunks, uint32_t max_chunks) {
   const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= T) return;
   const GridK& g = grid_of_tri<MULTI>(gs, t);
@@ -525,15 +527,15 @@ __global__ void k_seed(const __grid_constant__ GridSet gs, const TriRec* __restr
   seed_box(g, r, mn, ext);
   if (ext[0] <= 0 || ext[1] <= 0 || ext[2] <= 0) return;
   const unsigned long long total = (unsigned long long)ext[0] * ext[1] * ext[2];
-  if (split_box(t, total, 0u, 1u, &st->big_seeds, chunks)) return;
+  if (split_box(t, total, 0u, 1u, &st->big_seeds, chunks, max_chunks)) return;
   seed_cells<SIGN>(g, r, t, mn, ext, 0, total, keys, status, st);
 }
 
 template <int SIGN, bool MULTI>
 __global__ void k_seed_chunks(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris,
                               unsigned long long* keys, uint32_t* status, PropState* st,
-                              const uint2* __restrict__ chunks) {
-  const uint32_t n = min(st->big_seeds, kMaxChunks), warps = (gridDim.x * blockDim.x) >> 5;
+                              const uint2* __restrict__ chunks, uint32_t max_chunks) {
+  const uint32_t n = min(st->big_seeds, max_chunks), warps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
     const uint2 ch = chunks[i];
     if (ch.x == kNoChunk) continue;
@@ -1761,24 +1763,24 @@ __device__ __forceinline__ void ray_cells(const GridK& g, const TriRec& r, int j
 // One warp per (triangle, axis = blockIdx.y); large rectangles are split as in k_seed.
 template <int AXIS, bool MULTI, bool AUDIT>
 __device__ __forceinline__ void rays_of(const GridSet& gs, const TriRec* __restrict__ tris, uint32_t t, uint32_t* bits,
-                                        uint32_t* bits64, PropState* st, uint2* chunks) {
+                                        uint32_t* bits64, PropState* st, uint2* chunks, uint32_t max_chunks) {
   const GridK& g = grid_of_tri<MULTI>(gs, t);
   const TriRec r = tris[t];
   int j0, k0;
   uint32_t nk;
   unsigned long long total;
   if (!ray_box<AXIS>(g, r, &j0, &k0, &nk, &total)) return;
-  if (split_box(t, total, AXIS, 4u, &st->big_rays, chunks)) return;
+  if (split_box(t, total, AXIS, 4u, &st->big_rays, chunks, max_chunks)) return;
   ray_cells<AXIS, AUDIT>(g, r, j0, k0, nk, 0, total, bits, bits64, st);
 }
 template <bool MULTI, bool AUDIT>
 __global__ void k_rays(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t T, uint32_t* bits,
-                       PropState* st, uint32_t* bits64, uint2* chunks) {
+                       PropState* st, uint32_t* bits64, uint2* chunks, uint32_t max_chunks) {
   const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= T) return;
-  if (blockIdx.y == 0) rays_of<0, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks);
-  else if (blockIdx.y == 1) rays_of<1, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks);
-  else rays_of<2, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks);
+  if (blockIdx.y == 0) rays_of<0, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks, max_chunks);
+  else if (blockIdx.y == 1) rays_of<1, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks, max_chunks);
+  else rays_of<2, MULTI, AUDIT>(gs, tris, t, bits, bits64, st, chunks, max_chunks);
 }
 
 template <int AXIS, bool MULTI, bool AUDIT>
@@ -1795,8 +1797,9 @@ __device__ __forceinline__ void ray_chunk(const GridSet& gs, const TriRec* __res
 }
 template <bool MULTI, bool AUDIT>
 __global__ void k_ray_chunks(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t* bits,
-                             PropState* st, uint32_t* bits64, const uint2* __restrict__ chunks) {
-  const uint32_t n = min(st->big_rays, kMaxChunks), warps = (gridDim.x * blockDim.x) >> 5;
+                             PropState* st, uint32_t* bits64, const uint2* __restrict__ chunks,
+                             uint32_t max_chunks) {
+  const uint32_t n = min(st->big_rays, max_chunks), warps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
     const uint2 ch = chunks[i];
     if (ch.x == kNoChunk) continue;
@@ -1989,7 +1992,6 @@ struct GridJob::Impl {
   DevBuf<float> slack;
   bool filter = false;
   bool audit = false;          // FP64 audit (reports only)
-  DevBuf<uint2> chunks;        // pieces of large triangles (seeding, then rays)
   DevBuf<uint32_t> bits64;     // the audit's FP64-decided ray parities
 };
 
@@ -2015,7 +2017,7 @@ uint32_t GridJob::threads() const { return p->threads; }
 uint64_t GridJob::device_bytes() const {
   const Impl& J = *p;
   return J.comb_tris.n * sizeof(TriRec) + J.tri_grid.n * 4 + J.keys.n * 8 + J.bits.n * 4 +
-         J.chunks.n * sizeof(uint2) + J.bounds.n * sizeof(TriBound) + J.slack.n * 4 +
+         J.bounds.n * sizeof(TriBound) + J.slack.n * 4 +
          (uint64_t)kLists * J.cap * 8 + 2ull * J.cap * 4 + J.table.n * sizeof(GridK);
 }
 
@@ -2036,7 +2038,7 @@ uint32_t default_list_capacity(uint64_t cells) {
 uint64_t grid_job_bytes(uint64_t cells) {
   const uint64_t cap = default_list_capacity(cells);
   const uint64_t ray_words = 3 * (cells / 32 + 3 * std::cbrt((double)cells) * std::cbrt((double)cells));
-  return 8 * cells + (uint64_t)kLists * 8 * cap + 8 * cap + 4 * ray_words + (3u << 20);  // + 68 B per triangle
+  return 8 * cells + (uint64_t)kLists * 8 * cap + 8 * cap + 4 * ray_words + (1u << 20);  // + 68 B per triangle
 }
 
 int check_grid(const GridDesc& g) {
@@ -2144,7 +2146,6 @@ int GridJob::prepare(const MeshView* meshes, uint32_t n, const GridDesc* gds, in
   J.filter = tune.bound_filter;
   J.audit = tune.fp64_audit;
   if (tris && ((st = J.bounds.alloc(tris, s)) || (st = J.slack.alloc(tris, s)))) return st;
-  if (tris && (st = J.chunks.alloc(kMaxChunks, s))) return st;
   if (sign == M2S_SIGN_RAYCAST && (st = J.bits.alloc(woff, s))) return st;
   if (sign == M2S_SIGN_RAYCAST && J.audit && (st = J.bits64.alloc(woff, s))) return st;
   J.cap = tune.list_capacity ? tune.list_capacity : default_list_capacity(N);
@@ -2198,13 +2199,15 @@ int GridJob::enqueue(cudaStream_t s, cudaEvent_t* ev) {
                                                     J.bits.p, J.bits64.p, raycast ? J.ray_words : 0ull);
   ++J.launches;
   const unsigned chunk_blocks = 148u * 8u;
+  uint2* const chunks = J.lists.p;
+  const uint32_t max_chunks = (uint32_t)std::min<unsigned long long>((unsigned long long)kLists * J.cap, kMaxChunks);
   if (J.T > 0) {
     const unsigned sb = (unsigned)((J.T * 32ull + 255) / 256);
     auto seed = [&](auto sign_tag, auto multi_tag) {
       constexpr int S = decltype(sign_tag)::value;
       constexpr bool M = decltype(multi_tag)::value;
-      k_seed<S, M><<<sb, 256, 0, s>>>(J.gs, J.tris, J.T, J.keys.p, J.d_status, J.state.p, J.chunks.p);
-      k_seed_chunks<S, M><<<chunk_blocks, 256, 0, s>>>(J.gs, J.tris, J.keys.p, J.d_status, J.state.p, J.chunks.p);
+      k_seed<S, M><<<sb, 256, 0, s>>>(J.gs, J.tris, J.T, J.keys.p, J.d_status, J.state.p, chunks, max_chunks);
+      k_seed_chunks<S, M><<<chunk_blocks, 256, 0, s>>>(J.gs, J.tris, J.keys.p, J.d_status, J.state.p, chunks, max_chunks);
     };
     using Ray = std::integral_constant<int, M2S_SIGN_RAYCAST>;
     using Nor = std::integral_constant<int, M2S_SIGN_NORMAL>;
@@ -2251,8 +2254,8 @@ int GridJob::enqueue(cudaStream_t s, cudaEvent_t* ev) {
       const dim3 rb((unsigned)((J.T * 32ull + 255) / 256), 3);
       auto rays = [&](auto multi_tag, auto audit_tag) {
         constexpr bool M = decltype(multi_tag)::value, A = decltype(audit_tag)::value;
-        k_rays<M, A><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, J.bits64.p, J.chunks.p);
-        k_ray_chunks<M, A><<<chunk_blocks, 256, 0, s>>>(J.gs, J.tris, J.bits.p, J.state.p, J.bits64.p, J.chunks.p);
+        k_rays<M, A><<<rb, 256, 0, s>>>(J.gs, J.tris, J.T, J.bits.p, J.state.p, J.bits64.p, chunks, max_chunks);
+        k_ray_chunks<M, A><<<chunk_blocks, 256, 0, s>>>(J.gs, J.tris, J.bits.p, J.state.p, J.bits64.p, chunks, max_chunks);
       };
       if (J.audit) multi ? rays(std::true_type{}, std::true_type{}) : rays(std::false_type{}, std::true_type{});
       else multi ? rays(std::true_type{}, std::false_type{}) : rays(std::false_type{}, std::false_type{});
