@@ -250,7 +250,8 @@ int m2s_server_wait(m2s_server* server, uint64_t ticket, double timeout_s, int* 
 /* Frees a resident mesh that no queued or running request uses. */
 int m2s_server_remove_mesh(m2s_server* server, uint32_t mesh_id);
 /* [uploads, point requests, grid requests completed; failed; grid waves;
- *  grid requests in waves; most requests in one wave; reserved bytes; peak reserved bytes;
+ *  grid requests in waves; most requests in one wave; reserved bytes (with the resident
+ *  meshes' pillboxes, which take what the budget has to spare); peak of these;
  *  resident meshes; queued requests; evicted meshes]. */
 int m2s_server_stats(m2s_server* server, uint64_t out[12]);
 

@@ -70,7 +70,7 @@ struct MeshView {
   const TriRec* tris;    // crate triangle order
   const TriRec* stris;   // LBVH leaf order
   const BvhNode* nodes;  // n_tris - 1 internal nodes (node 0 is the root)
-  const Pill* pills;     // two per internal node
+  const Pill* pills;     // two per internal node, or NULL (the nodes' limits are then 0)
   uint32_t n_tris;
   uint32_t root;  // 0, or LEAF_BIT | 0 for a single triangle
 };
@@ -133,11 +133,15 @@ struct MeshInput {
 struct DeviceMesh {
   DevBuf<TriRec> tris, stris;
   DevBuf<BvhNode> nodes;
-  DevBuf<Pill> pills;
+  DevBuf<Pill> pills;  // none where memory did not suffice or the server gave them back
   uint32_t n_tris = 0;
   uint32_t root = 0;
   MeshView view() const { return {tris.p, stris.p, nodes.p, pills.p, n_tris, root}; }
 };
+
+// Gives the pillboxes of a mesh that no search reads back; searches then prune
+// by the boxes alone, with the same results.  Waits for the stream.
+int drop_pills(DeviceMesh* m, cudaStream_t s);
 
 // Builds the triangle records and the LBVH.  d_status receives status bits.
 // with_tree = false builds the triangle records only (grid path, brute force).

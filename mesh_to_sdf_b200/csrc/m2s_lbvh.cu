@@ -157,6 +157,12 @@ __global__ void k_karras(const uint32_t* __restrict__ keys, int n, BvhNode* node
   if (right & LEAF_BIT) leaf_parent[gamma + 1] = i;
   else node_parent[gamma + 1] = i;
   if (i == 0) node_parent[0] = 0xFFFFFFFFu;
+  nodes[i].r_lo.w = nodes[i].r_hi.w = 0.0f;  // no pillboxes (k_pills)
+}
+
+__global__ void k_no_pills(BvhNode* nodes, uint32_t n) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) nodes[i].r_lo.w = nodes[i].r_hi.w = 0.0f;
 }
 
 __global__ void k_gather_leaves(const TriRec* __restrict__ tris, const uint32_t* __restrict__ perm, int n,
@@ -342,6 +348,15 @@ inline unsigned grid_for(uint64_t n, int threads = kThreads) { return (unsigned)
 
 }  // namespace
 
+int drop_pills(DeviceMesh* m, cudaStream_t s) {
+  if (!m->pills.p) return M2S_OK;
+  k_no_pills<<<grid_for(m->nodes.n), kThreads, 0, s>>>(m->nodes.p, (uint32_t)m->nodes.n);
+  M2S_CUDA(cudaGetLastError());
+  M2S_CUDA(cudaStreamSynchronize(s));
+  m->pills.release();
+  return M2S_OK;
+}
+
 int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, cudaStream_t s, bool with_tree) {
   if (in.n_tris > 0x7FFFFFFFull) return M2S_ERR_INVALID_ARGUMENT;
   const uint32_t T = (uint32_t)in.n_tris;
@@ -369,16 +384,19 @@ int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, 
   if (T < 2) return M2S_OK;
   DevBuf<uint32_t> node_parent, leaf_parent, counters;
   DevBuf<uint2> range;
-  if ((st = out->nodes.alloc(T - 1, s)) || (st = out->pills.alloc(2ull * (T - 1), s)) || (st = range.alloc(T - 1, s)) || (st = node_parent.alloc(T - 1, s)) || (st = leaf_parent.alloc(T, s)) ||
-      (st = counters.alloc(T - 1, s)))
+  if ((st = out->nodes.alloc(T - 1, s)) || (st = node_parent.alloc(T - 1, s)) || (st = leaf_parent.alloc(T, s)) ||
+      (st = counters.alloc(T - 1, s)) || (st = range.alloc(T - 1, s)))
     return st;
+  // (pillboxes only make searches faster: a mesh whose tree just fits goes without)
+  if (out->pills.alloc(2ull * (T - 1), s)) cudaGetLastError();
   M2S_CUDA(cudaMemsetAsync(counters.p, 0, (T - 1) * sizeof(uint32_t), s));
   k_karras<<<grid_for(T - 1), kThreads, 0, s>>>(keys.p, (int)T, out->nodes.p, node_parent.p, leaf_parent.p,
                                           range.p);
   M2S_CUDA(cudaGetLastError());
   k_refit<<<grid_for(T), kThreads, 0, s>>>(boxes.p, perm.p, (int)T, out->nodes.p, node_parent.p, leaf_parent.p,
                                            counters.p);
-  k_pills<<<grid_for(2ull * (T - 1), 128), 128, 0, s>>>(out->stris.p, out->nodes.p, range.p, 2u * (T - 1), out->pills.p);
+  if (out->pills.p)
+    k_pills<<<grid_for(2ull * (T - 1), 128), 128, 0, s>>>(out->stris.p, out->nodes.p, range.p, 2u * (T - 1), out->pills.p);
   M2S_CUDA(cudaGetLastError());
   return M2S_OK;
 }

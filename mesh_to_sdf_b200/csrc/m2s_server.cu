@@ -27,6 +27,13 @@
 // reservation fits.  A request that could never fit is refused with
 // M2S_ERR_OUT_OF_MEMORY.  An upload that does not fit first evicts resident
 // meshes that no queued or running request uses, least recently used first.
+//
+// Pillboxes (64 bytes a triangle that only make point searches faster) take
+// what the budget has to spare: no request is refused, delayed behind idle
+// memory or answered by an eviction because of them.  They are counted beside
+// the reservations, and when a reservation needs their room, meshes that no
+// request runs on give theirs back, least recently used first; those that one
+// runs on are waited for.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -70,6 +77,7 @@ struct Request {
   int grid_sign = 0;
   float* out = nullptr;
   uint64_t cells = 0;
+  bool running = false;  // counted in its mesh's running
   Clock::time_point t_submit, t_done;
   int status = -1;  // -1 while pending
 };
@@ -80,14 +88,17 @@ struct MeshEntry {
   uint64_t bytes = 0;
   uint64_t last_use = 0;
   int users = 0;  // queued or running requests
+  int running = 0;  // running ones
+  uint64_t pills = 0;  // bytes of its pillboxes, in m2s_server::spare
   bool failed = false;
 };
 
-// Device bytes a resident mesh holds: triangle records in both orders (48 B
-// each), 64-byte LBVH nodes and 64 bytes of pillboxes a node; the build needs about as much again for a
-// moment (vertices, indices, Morton keys, sort buffers).
+// Device bytes a resident mesh holds, pillboxes apart: triangle records in both
+// orders (48 B each) and 64-byte LBVH nodes.  The build needs less than as much
+// again for a moment: 64 bytes a triangle of pillboxes, 60 of boxes, Morton keys
+// and links, beside vertices and indices.
 uint64_t mesh_bytes(uint64_t tris, int accel) {
-  return accel == M2S_ACCEL_NONE ? 48 * tris : 224 * tris;
+  return accel == M2S_ACCEL_NONE ? 48 * tris : 160 * tris;
 }
 uint64_t upload_bytes(uint64_t tris, uint64_t nv, uint64_t ni, int bits, int accel) {
   return 2 * mesh_bytes(tris, accel) + 12 * nv + ni * (bits / 8) + (1u << 20);
@@ -137,30 +148,51 @@ struct m2s_server {
   uint64_t next_ticket = 1;
   uint32_t next_mesh = 1;
   uint64_t reserved = 0, peak = 0, clock = 0;
+  uint64_t spare = 0;  // bytes of the resident meshes' pillboxes
+  uint64_t busy = 0;   // of them, those of meshes with a running request
   std::map<uint64_t, RequestP> tickets;
   std::map<uint32_t, MeshEntry> meshes;
   std::deque<RequestP> q[3];
   // counters
   uint64_t completed[3] = {0, 0, 0}, failed = 0, grid_batches = 0, grid_batched = 0, max_batch = 0, evictions = 0;
 
-  cudaStream_t s_upload = nullptr, s_grid[kGridLanes] = {};
+  cudaStream_t s_upload = nullptr, s_trim = nullptr, s_grid[kGridLanes] = {};
   std::vector<cudaStream_t> s_points;
   std::thread th[2 + kGridLanes];  // uploads, points, grid lanes
   bool lane_busy[kGridLanes] = {};  // a lane runs a wave
 
   // ---- helpers (mu held) ----
   bool fits(uint64_t need) const { return reserved + need <= budget; }
+  // `need` fits beside the pillboxes that running requests read.
+  bool admits(uint64_t need) const { return reserved + need + busy <= budget; }
   // The head of queue k can be taken now: its mesh is gone or failed (it
   // completes with an error), or its mesh is resident and it fits.
   bool head_ready(int k) const {
     if (q[k].empty()) return false;
     const RequestP& r = q[k].front();
     auto it = meshes.find(r->mesh_id);
-    return it == meshes.end() || it->second.failed || (it->second.mesh && fits(r->need));
+    return it == meshes.end() || it->second.failed || (it->second.mesh && admits(r->need));
   }
   void reserve(uint64_t need) {
     reserved += need;
-    peak = std::max(peak, reserved);
+    while (reserved + spare > budget) {  // pillboxes give way
+      MeshEntry* victim = nullptr;
+      for (auto& kv : meshes)
+        if (kv.second.pills && !kv.second.running && (!victim || kv.second.last_use < victim->last_use))
+          victim = &kv.second;
+      // (no search reads them: no request runs on the mesh)
+      if (!victim || drop_pills(&victim->mesh->mesh, s_trim)) break;
+      spare -= victim->pills;
+      victim->pills = 0;
+    }
+    peak = std::max(peak, reserved + spare);
+  }
+  // A request leaves its queue for the mesh it needs.
+  void start(const RequestP& r, MeshEntry& e) {
+    reserve(r->need);
+    r->running = true;
+    if (e.running++ == 0) busy += e.pills;
+    e.last_use = ++clock;
   }
   void finish(const RequestP& r, int status) {
     r->status = status;
@@ -169,7 +201,10 @@ struct m2s_server {
     r->need = 0;
     if (r->kind != kUpload) {
       auto it = meshes.find(r->mesh_id);
-      if (it != meshes.end()) it->second.users--;
+      if (it != meshes.end()) {
+        it->second.users--;
+        if (r->running && --it->second.running == 0) busy -= it->second.pills;
+      }
     }
     if (status == M2S_OK) completed[r->kind]++;
     else failed++;
@@ -190,6 +225,7 @@ struct m2s_server {
       MeshEntry e = meshes[victim];
       meshes.erase(victim);
       reserved -= e.bytes;
+      spare -= e.pills;
       delete e.mesh;  // nothing queued or running uses it; its buffers go back on the upload stream
       ++evictions;
     }
@@ -214,7 +250,7 @@ void m2s_server::upload_loop() {
       // release memory (the request fits the budget, checked at submit).
       for (;;) {
         evict_for(r->need);
-        if (fits(r->need) || stop) break;
+        if (admits(r->need) || stop) break;
         cv_work.wait(lk);
       }
       if (stop) return;
@@ -238,6 +274,11 @@ void m2s_server::upload_loop() {
       e.failed = true;
     }
     finish(r, st);
+    if (st == M2S_OK) {
+      const uint64_t pills = h->mesh.pills.n * sizeof(Pill);
+      spare += e.pills = h->mesh.pills.p ? pills : 0;
+      reserve(0);  // keeps them, or others', as far as they fit
+    }
   }
 }
 
@@ -283,10 +324,9 @@ void m2s_server::points_loop() {
           finish(r, M2S_ERR_INVALID_ARGUMENT);
           continue;
         }
-        if (!it->second.mesh || !fits(r->need)) break;
+        if (!it->second.mesh || !admits(r->need)) break;
         q[kPoints].pop_front();
-        reserve(r->need);
-        it->second.last_use = ++clock;
+        start(r, it->second);
         go.emplace_back(r, it->second.mesh);
       }
     }
@@ -384,12 +424,11 @@ void m2s_server::grid_loop(int lane) {
           finish(r, M2S_ERR_INVALID_ARGUMENT);
           continue;
         }
-        if (!it->second.mesh || !fits(r->need)) break;
+        if (!it->second.mesh || !admits(r->need)) break;
         if (!wave.empty() && r->grid_sign != wave.front()->grid_sign) break;  // one sign per wave
         if (!wave.empty() && cells + r->cells > tune.wave_cells) break;
         q[kGrid].pop_front();
-        reserve(r->need);
-        it->second.last_use = ++clock;
+        start(r, it->second);
         wave.push_back(r);
         views.push_back(it->second.mesh->mesh.view());
         cells += r->cells;
@@ -481,7 +520,8 @@ int m2s_server_create(uint64_t hbm_budget_bytes, uint32_t point_streams, m2s_ser
   cudaGetDevice(&S->device);
   S->budget = hbm_budget_bytes;
   S->n_streams = std::max<uint32_t>(1, std::min<uint32_t>(point_streams ? point_streams : 4, 32));
-  bool ok = cudaStreamCreateWithFlags(&S->s_upload, cudaStreamNonBlocking) == cudaSuccess;
+  bool ok = cudaStreamCreateWithFlags(&S->s_upload, cudaStreamNonBlocking) == cudaSuccess &&
+            cudaStreamCreateWithPriority(&S->s_trim, cudaStreamNonBlocking, -1) == cudaSuccess;
   for (int l = 0; ok && l < kGridLanes; ++l)
     ok = cudaStreamCreateWithFlags(&S->s_grid[l], cudaStreamNonBlocking) == cudaSuccess;
   for (uint32_t i = 0; ok && i < S->n_streams; ++i) {
@@ -493,6 +533,7 @@ int m2s_server_create(uint64_t hbm_budget_bytes, uint32_t point_streams, m2s_ser
     st = cuda_fail(cudaGetLastError(), "cudaStreamCreateWithFlags");
     for (auto s : S->s_points) cudaStreamDestroy(s);
     if (S->s_upload) cudaStreamDestroy(S->s_upload);
+    if (S->s_trim) cudaStreamDestroy(S->s_trim);
     for (auto g : S->s_grid)
       if (g) cudaStreamDestroy(g);
     delete S;
@@ -535,6 +576,7 @@ void m2s_server_free(m2s_server* S) {
   cudaStreamSynchronize(S->s_upload);
   for (auto s : S->s_points) cudaStreamDestroy(s);
   cudaStreamDestroy(S->s_upload);
+  cudaStreamDestroy(S->s_trim);
   for (auto g : S->s_grid) cudaStreamDestroy(g);
   cudaSetDevice(prev);
   delete S;
@@ -639,6 +681,7 @@ int m2s_server_remove_mesh(m2s_server* S, uint32_t mesh_id) {
   auto it = S->meshes.find(mesh_id);
   if (it == S->meshes.end() || !it->second.mesh || it->second.users) return M2S_ERR_INVALID_ARGUMENT;
   S->reserved -= it->second.bytes;
+  S->spare -= it->second.pills;
   delete it->second.mesh;
   S->meshes.erase(it);
   S->cv_work.notify_all();
@@ -652,7 +695,7 @@ int m2s_server_stats(m2s_server* S, uint64_t out[12]) {
   for (auto& kv : S->meshes) resident += kv.second.mesh ? 1 : 0;
   for (auto& qq : S->q) queued += qq.size();
   const uint64_t v[12] = {S->completed[kUpload], S->completed[kPoints], S->completed[kGrid], S->failed,
-                          S->grid_batches,       S->grid_batched,       S->max_batch,        S->reserved,
+                          S->grid_batches,       S->grid_batched,       S->max_batch,        S->reserved + S->spare,
                           S->peak,               resident,              queued,              S->evictions};
   for (int i = 0; i < 12; ++i) out[i] = v[i];
   return M2S_OK;
