@@ -299,6 +299,13 @@ int m2s_check_mesh_triangle_list(const float* vertices, uint64_t n_vertices, con
 int m2s_radix_sort_pairs_device(uint32_t* d_keys, uint32_t* d_values, uint64_t n, int key_bits,
                                 void* stream);
 
+/* Diagnostics of that sort (no counterpart in the reference): the same with
+ * another limit of the polls after which a tile counts the digits before it
+ * from the keys (the sort's own is 65,536; 0 makes every tile count) and, with
+ * wide_words != 0, the 64-bit counts that 2^30 pairs and more take. */
+int m2s_test_radix_sort(uint32_t* d_keys, uint32_t* d_values, uint64_t n, int key_bits,
+                        uint32_t max_polls, int wide_words, void* stream);
+
 /* Diagnostics of the last grid call on this thread: [seed updates, relax
  * rounds, states relaxed, neighbour proposals (the on-grid cells of the 26
  * around each relaxed state; a proposal dropped unevaluated, see

@@ -48,6 +48,7 @@ SIGNATURES = {
     "m2s_last_query_audit": (I, [P]),
     "m2s_grid_plan_waves": (ctypes.c_uint32, [P]),
     "m2s_radix_sort_pairs_device": (I, [P, P, U64, I, P]),
+    "m2s_test_radix_sort": (I, [P, P, U64, I, ctypes.c_uint32, I, P]),
     "m2s_sort_cells_by_distance_device": (I, [P, U64, P, P, P]),
     "m2s_sort_cells_by_distance": (I, [P, U64, P, P, P]),
     "m2s_serialize_generic": (I, [P, U64, P, U64, P, U64, P]),

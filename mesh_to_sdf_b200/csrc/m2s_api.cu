@@ -562,4 +562,12 @@ int m2s_radix_sort_pairs_device(uint32_t* d_keys, uint32_t* d_values, uint64_t n
   return radix_sort_pairs(d_keys, d_values, n, key_bits, (cudaStream_t)stream);
 }
 
+int m2s_test_radix_sort(uint32_t* d_keys, uint32_t* d_values, uint64_t n, int key_bits, uint32_t max_polls,
+                        int wide_words, void* stream) {
+  int st;
+  if ((st = require_device())) return st;
+  if (n && (!d_keys || !d_values)) return M2S_ERR_INVALID_ARGUMENT;
+  return radix_sort_pairs_with(d_keys, d_values, n, key_bits, max_polls, wide_words != 0, (cudaStream_t)stream);
+}
+
 }  // extern "C"

@@ -154,6 +154,11 @@ int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, 
 // keep_keys = false leaves the keys in no order (the values alone are wanted).
 int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, cudaStream_t s, bool keep_keys = true);
 
+// The same with another limit of the look-back's polls (0: every count from the
+// keys) and, with big, the 64-bit tile words of 2^30 pairs and more (tests).
+int radix_sort_pairs_with(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, uint32_t max_polls, bool big,
+                          cudaStream_t s);
+
 // order: 0 .. n - 1 stably by f32::total_cmp of d; minmax (2 floats, may be
 // NULL): the extremes of the values that are no NaN.
 int sort_floats(const float* d, uint64_t n, uint32_t* order, float* minmax, cudaStream_t s);

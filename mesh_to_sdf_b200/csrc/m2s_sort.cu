@@ -11,13 +11,17 @@
 // a block waits for have started before it.  A wait is bounded all the same:
 // past its limit the thread counts its digit in the tiles before it from the
 // keys themselves (a pass never overwrites its input), slower but the same sum.
+// (The look-back is Merrill and Garland's, "Single-pass Parallel Prefix Scan with
+// Decoupled Look-back", 2016; one kernel a digit with it is Adinets and Merrill's
+// "Onesweep", 2022.)
 //
 // Bound: HBM, 16 bytes a pair and pass (8 read, 8 written).  Before, each pass
 // read the keys again for per-tile counts, scanned 256 counts a tile in three
 // launches and ranked a tile in eight steps of three block barriers: 16.7M
 // pairs 176 us a pass in the scatter alone, 20 launches a sort; now 132 us a
-// pass (2.0 TB/s: the tiles' chain of loads, ranks and totals, about 10 us with
-// two tiles an SM, sets the time) and 5 launches: the sort 1.08 -> 0.57 ms.
+// pass (2.0 TB/s: 2,048 tiles, two an SM at a time, are seven waves of about
+// 19 us, a tile's chain of loads, ranks and totals) and 5 launches: the sort
+// 1.08 -> 0.57 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -160,7 +164,7 @@ __device__ __forceinline__ void st_word(uint32_t* p, uint32_t v) {
 __device__ __forceinline__ void st_word(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-constexpr uint32_t kPolls = 1u << 16;  // in vain (some 50 ms; a tile takes microseconds)
+constexpr uint32_t kPolls = 1u << 16;  // in vain, at most (some 50 ms; a tile takes microseconds)
 constexpr uint32_t kAhead = 8;
 
 // The lanes of the warp whose d (9 bits) is this lane's, by a ballot per bit
@@ -185,7 +189,8 @@ template <int THREADS, int ITEMS, class Source, class Word, bool KEYS_OUT>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_sort_pass(Source src, uint32_t* __restrict__ kout,
                                                                        uint32_t* __restrict__ vout, uint64_t n,
                                                                        int shift, const uint32_t* __restrict__ first,
-                                                                       Word* words, uint32_t* next_tile) {
+                                                                       Word* words, uint32_t* next_tile,
+                                                                       uint32_t max_polls) {
   using W = TileWord<Word>;
   constexpr int kTile = THREADS * ITEMS, kTileWarps = THREADS / 32;
   extern __shared__ uint32_t s_mem[];
@@ -267,6 +272,11 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_sort_pass(Source sr
     uint64_t before = 0;
     uint32_t polls = 0;
     for (uint32_t j = tile; j > 0;) {
+      if (polls == max_polls) {  // gave up: count tiles 0 .. j - 1
+        const uint64_t end = (uint64_t)j * kTile;
+        for (uint64_t i = 0; i < end; ++i) before += ((src.key(i) >> shift) & 0xFFu) == d ? 1u : 0u;
+        break;
+      }
       Word w[kAhead];
 #pragma unroll
       for (uint32_t a = 0; a < kAhead; ++a)
@@ -282,11 +292,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_sort_pass(Source sr
       }
       if (found) break;
       j -= taken;
-      if (taken == 0 && ++polls == kPolls) {  // gave up: count tiles 0 .. j - 1
-        const uint64_t end = (uint64_t)j * kTile;
-        for (uint64_t i = 0; i < end; ++i) before += ((src.key(i) >> shift) & 0xFFu) == d ? 1u : 0u;
-        break;
-      }
+      if (taken == 0) ++polls;
     }
     if (tile != 0) st_word(row, W::kTotal | (Word)(before + total));
     dest[d] = first[d] + (uint32_t)before - in_tile;
@@ -313,8 +319,9 @@ struct SortPlan {
   uint64_t tiles = 0;
   bool big = false;   // counts that need 64-bit words
   bool wide = false;  // large tiles
+  uint32_t max_polls = kPolls;
   int init(uint64_t n, int passes, cudaStream_t s) {
-    big = n >= (1ull << 30);
+    big = big || n >= (1ull << 30);
     wide = n >= kLargeMin;
     const uint64_t tile = (big || wide) ? kLargeThreads * kLargeItems : kSmallThreads * kSmallItems;
     tiles = (n + tile - 1) / tile;
@@ -333,7 +340,7 @@ struct SortPlan {
     if (smem > 48 * 1024 - 2048) M2S_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     kern<<<(unsigned)tiles, THREADS, smem, s>>>(src, kout, vout, n, 8 * p, st->hist[p],
                                                 reinterpret_cast<Word*>(words) + (uint64_t)p * tiles * kDigits,
-                                                &st->tiles[p]);
+                                                &st->tiles[p], max_polls);
     M2S_CUDA(cudaGetLastError());
     return M2S_OK;
   }
@@ -351,11 +358,12 @@ unsigned count_blocks(uint64_t n) {
 
 }  // namespace
 
-int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, cudaStream_t s, bool keep_keys) {
+namespace {
+int sort_pairs(SortPlan& plan, uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, cudaStream_t s,
+               bool keep_keys) {
   if (n <= 1) return M2S_OK;
   if (key_bits <= 0 || key_bits > 32 || n > 0xFFFFFFFFull) return M2S_ERR_INVALID_ARGUMENT;
   const int passes = (key_bits + 7) / 8;
-  SortPlan plan;
   DevBuf<uint32_t> k2, v2;
   int r;
   if ((r = plan.init(n, passes, s)) || (r = k2.alloc(n, s)) || (r = v2.alloc(n, s))) return r;
@@ -382,6 +390,21 @@ int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, c
     M2S_CUDA(cudaMemcpyAsync(vals, va, n * 4, cudaMemcpyDeviceToDevice, s));
   }
   return M2S_OK;
+}
+
+}  // namespace
+
+int radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, cudaStream_t s, bool keep_keys) {
+  SortPlan plan;
+  return sort_pairs(plan, keys, vals, n, key_bits, s, keep_keys);
+}
+
+int radix_sort_pairs_with(uint32_t* keys, uint32_t* vals, uint64_t n, int key_bits, uint32_t max_polls, bool big,
+                          cudaStream_t s) {
+  SortPlan plan;
+  plan.max_polls = max_polls;
+  plan.big = big;
+  return sort_pairs(plan, keys, vals, n, key_bits, s, true);
 }
 
 int sort_floats(const float* d, uint64_t n, uint32_t* order, float* minmax, cudaStream_t s) {

@@ -135,6 +135,8 @@ extern "C" {
     // ---- utilities and diagnostics
     pub fn m2s_radix_sort_pairs_device(d_keys: *mut u32, d_values: *mut u32, n: u64, key_bits: c_int,
                                        stream: *mut c_void) -> c_int;
+    pub fn m2s_test_radix_sort(d_keys: *mut u32, d_values: *mut u32, n: u64, key_bits: c_int, max_polls: u32,
+                               wide_words: c_int, stream: *mut c_void) -> c_int;
     pub fn m2s_last_grid_stats(out: *mut u64) -> c_int;
     pub fn m2s_last_grid_filter_stats(out: *mut u64) -> c_int;
     pub fn m2s_set_profiling(enable: c_int);
