@@ -200,7 +200,7 @@ bool profiling_enabled();
 // [queries, the four traversal counts, the seven FP64-audit counts]
 void record_query_stats(const uint64_t stats[12]);
 
-// allow_alloc = false keeps the brute force in one pass with no scratch buffer.
+// allow_alloc = false takes no scratch buffer: d_out then holds what chunks merge.
 int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, float* d_out,
                     uint32_t* d_status, cudaStream_t s, bool allow_alloc = true);
 
