@@ -1773,8 +1773,12 @@ __device__ __forceinline__ void rays_of(const GridSet& gs, const TriRec* __restr
   if (split_box(t, total, AXIS, 4u, &st->big_rays, chunks, max_chunks)) return;
   ray_cells<AXIS, AUDIT>(g, r, j0, k0, nk, 0, total, bits, bits64, st);
 }
+// Bound: latency (record, grid, rectangle and bit words one after another), so
+// warps in flight count: six blocks an SM, five for batches (48 registers); at the
+// 52 that the three axes in one kernel take by themselves four fit (12 grids,
+// 296,000 triangles: 292 us as three launches, 327 with 52, 290 now).
 template <bool MULTI, bool AUDIT>
-__global__ void k_rays(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t T, uint32_t* bits,
+__global__ void __launch_bounds__(256, AUDIT ? 3 : (MULTI ? 5 : 6)) k_rays(const __grid_constant__ GridSet gs, const TriRec* __restrict__ tris, uint32_t T, uint32_t* bits,
                        PropState* st, uint32_t* bits64, uint2* chunks, uint32_t max_chunks) {
   const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= T) return;
