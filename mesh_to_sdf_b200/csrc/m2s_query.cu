@@ -32,6 +32,10 @@ constexpr float F32_MAX = 3.40282347e+38f;
 __device__ __forceinline__ float pill_query_slack(P3 p) {
   return kPillSlack * fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z)));
 }
+__device__ __forceinline__ TriRec load_tri(const TriRec* t, uint32_t i) {
+  const float4* f = reinterpret_cast<const float4*>(t + i);
+  return {__ldg(f), __ldg(f + 1), __ldg(f + 2)};
+}
 __device__ __forceinline__ P3 load_query(const float* q, uint64_t i) { return {q[3 * i], q[3 * i + 1], q[3 * i + 2]}; }
 
 // ---------------------------------------------------------------------------
@@ -74,7 +78,15 @@ constexpr int kBfTile = 256;  // triangles per stage: 256 * 48 B = 12 KiB
 // there and let small meshes spread over more blocks (1,280 triangles, 1,000
 // points 0.125 -> 0.082 ms).
 constexpr int kBrThreads = 256;
-constexpr int kBrTile = 64;  // triangles per stage
+constexpr int kBrTile = 64;  // triangles per stage, at most
+// Triangles per stage of a call: fewer where the tiles of 64 would leave SMs
+// idle, since a block's time is its tiles' one after another (1,000 queries on 80 /
+// 320 / 1,280 triangles: tiles of 64 95 / 83 / 78 us, now 29 / 30 / 33).
+inline uint32_t brute_tile(uint32_t n_tris, uint32_t blocks) {
+  uint32_t tile = kBrTile;
+  while (tile > 8 && (uint64_t)blocks * ((n_tris + tile - 1) / tile) < 2 * 148) tile /= 2;
+  return tile;
+}
 
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
@@ -121,7 +133,7 @@ __global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* _
                                                               const float* __restrict__ q, uint64_t nq,
                                                               float* __restrict__ out, uint32_t* status,
                                                               uint2* __restrict__ part,
-                                                              const uint32_t* __restrict__ order) {
+                                                              const uint32_t* __restrict__ order, uint32_t stage) {
   __shared__ __align__(128) TriRec tile[2][kBrTile];
   __shared__ BrutePair pair[kBrTile];
   __shared__ __align__(8) uint64_t bar[2];
@@ -137,12 +149,12 @@ __global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* _
   }
   const f32x2 px = pack2(p[0].x, p[1].x), py = pack2(p[0].y, p[1].y), pz = pack2(p[0].z, p[1].z);
   // this block's chunk of triangles: whole tiles [t_begin, t_end)
-  const uint32_t all_tiles = (T + kBrTile - 1) / kBrTile;
+  const uint32_t all_tiles = (T + stage - 1) / stage;  // stage: brute_tile
   const uint32_t per = (all_tiles + gridDim.y - 1) / gridDim.y;
   const uint32_t t_begin = min(all_tiles, blockIdx.y * per), t_end = min(all_tiles, t_begin + per);
   const uint32_t ntile = t_end - t_begin;
-  tris += (uint64_t)t_begin * kBrTile;
-  T = ntile == 0 ? 0u : (t_end == all_tiles ? T - t_begin * kBrTile : ntile * kBrTile);
+  tris += (uint64_t)t_begin * stage;
+  T = ntile == 0 ? 0u : (t_end == all_tiles ? T - t_begin * stage : ntile * stage);
 
   if (tid == 0) {
     mbar_init(&bar[0], 1);
@@ -151,10 +163,10 @@ __global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* _
   }
   __syncthreads();
   auto issue = [&](uint32_t i) {
-    uint32_t cnt = min((uint32_t)kBrTile, T - i * kBrTile);
+    uint32_t cnt = min(stage, T - i * stage);
     uint32_t bytes = cnt * (uint32_t)sizeof(TriRec);
     mbar_arrive_expect_tx(&bar[i & 1], bytes);
-    bulk_g2s(&tile[i & 1][0], tris + (uint64_t)i * kBrTile, bytes, &bar[i & 1]);
+    bulk_g2s(&tile[i & 1][0], tris + (uint64_t)i * stage, bytes, &bar[i & 1]);
   };
   if (tid == 0) {
     if (ntile > 0) issue(0);
@@ -172,7 +184,7 @@ __global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* _
   for (uint32_t i = 0; i < ntile; ++i) {
     const int buf = i & 1;
     if (!mbar_wait_bounded(&bar[buf], (i >> 1) & 1)) lost = true;
-    const uint32_t cnt = min((uint32_t)kBrTile, T - i * kBrTile);
+    const uint32_t cnt = min(stage, T - i * stage);
     const TriRec* tl = tile[buf];
     lost = __syncthreads_or(lost);  // pairs are only formed from a tile every thread has
     if (!lost && tid < (int)cnt) {
@@ -295,6 +307,37 @@ __global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* _
     const float d = fminf(F32_MAX, fsqrt(best[u]));
     out[qi[u]] = (hits[u] & 1u) ? -d : d;
   }
+}
+
+// Raycast against few triangles: a thread per query over all of them.  Launches
+// and a chain of distances set the time, so there is nothing to split or to skip,
+// and the closest point is the one without branches (a warp's queries lie in
+// different regions).  In us, one query a thread with planes (the kernel before the
+// packed one) / packed with tiles of 64 / packed with brute_tile / this one: 20
+// triangles, 1,000 queries 26 / 45 / 34 / 22; 44, 100,000 50 / 78 / 73 / 42; 80,
+// 30,000 56 / 98 / 45 / 52, 100,000 82 / 123 / 119 / 75, 500,000 316 / 230 / 230 / 310;
+// 194, 50,000 115 / 124 / 123 / 111, 200,000 282 / 258 / 257 / 285.
+inline bool brute_few(uint32_t n_tris, uint64_t nq) {
+  return n_tris * nq < 1ull << 25 && (n_tris <= 48 || (n_tris <= 224 && nq >= 49152));
+}
+__global__ void __launch_bounds__(128) k_brute_raycast_few(const TriRec* __restrict__ tris, uint32_t T,
+                                                           const float* __restrict__ q, uint64_t nq,
+                                                           float* __restrict__ out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nq) return;
+  const P3 p = load_query(q, i);
+  float best = INFINITY;
+  uint32_t hits = 0;
+#pragma unroll 2
+  for (uint32_t t = 0; t < T; ++t) {
+    const TriRec r = load_tri(tris, t);
+    const P3 a = p3(r.a), b = p3(r.b), c = p3(r.c);
+    best = fminf(best, point_triangle_distance2_sel(p, a, b, c, __float_as_int(r.a.w)));  // a NaN distance is ignored
+    float tt;
+    hits += ray_hit_aligned<0>(p, a, b, c, &tt) ? 1u : 0u;
+  }
+  const float d = fminf(F32_MAX, fsqrt(best));
+  out[i] = (hits & 1u) ? -d : d;
 }
 
 // Normal, one thread per query: compare_distances folded over all triangles in
@@ -471,11 +514,6 @@ __device__ __forceinline__ BvhNode load_node(const BvhNode* nodes, uint32_t i) {
   n.r_lo = __ldg(f + 2);
   n.r_hi = __ldg(f + 3);
   return n;
-}
-
-__device__ __forceinline__ TriRec load_tri(const TriRec* t, uint32_t i) {
-  const float4* f = reinterpret_cast<const float4*>(t + i);
-  return {__ldg(f), __ldg(f + 1), __ldg(f + 2)};
 }
 
 // The pillbox bound (Pill, m2s_internal.cuh): a squared distance that no
@@ -1558,7 +1596,8 @@ int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, 
   DevBuf<uint32_t> keys, order;
   DevBuf<int> bounds;
   const uint32_t* ord = nullptr;
-  const bool thread_kernel = sign == M2S_SIGN_RAYCAST || nq >= kBruteWarpMaxQueries;
+  const bool few = sign == M2S_SIGN_RAYCAST && brute_few(m.n_tris, nq);
+  const bool thread_kernel = !few && (sign == M2S_SIGN_RAYCAST || nq >= kBruteWarpMaxQueries);
   if (allow_alloc && thread_kernel && nq >= 1024 && nq <= 0xFFFFFFFFull && nq * m.n_tris >= kBruteSortMinPairs) {
     int st;
     if ((st = keys.alloc(nq, s)) || (st = order.alloc(nq, s)) || (st = bounds.alloc(6, s))) return st;
@@ -1569,10 +1608,12 @@ int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, 
     if ((st = radix_sort_pairs(keys.p, order.p, nq, 30, s, /*keep_keys=*/false))) return st;
     ord = order.p;
   }
-  if (sign == M2S_SIGN_RAYCAST) {
+  if (few) {
+    k_brute_raycast_few<<<(unsigned)((nq + 127) / 128), 128, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out);
+  } else if (sign == M2S_SIGN_RAYCAST) {
     // Enough (query, triangle chunk) blocks to fill the GPU ~4 deep.
     const unsigned blocks = (unsigned)((nq + 2 * kBrThreads - 1) / (2 * kBrThreads));
-    const uint32_t tiles = (m.n_tris + kBrTile - 1) / kBrTile;
+    const uint32_t stage = brute_tile(m.n_tris, blocks), tiles = (m.n_tris + stage - 1) / stage;
     uint32_t chunks = (uint32_t)std::max<uint64_t>(1, (148ull * 16ull + blocks - 1) / blocks);
     chunks = std::max(1u, std::min(chunks, std::min(tiles, 256u)));
     DevBuf<uint2> part;
@@ -1580,7 +1621,8 @@ int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, 
     if (chunks > 1 && allow_alloc && (st = part.alloc(nq, s))) return st;
     const unsigned fb = (unsigned)std::min<uint64_t>((nq + 255) / 256, 148u * 16u);
     if (chunks > 1) k_brute_init<<<fb, 256, 0, s>>>(part.p, d_out, nq);
-    k_brute_raycast<<<dim3(blocks, chunks), kBrThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out, d_status, part.p, ord);
+    k_brute_raycast<<<dim3(blocks, chunks), kBrThreads, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out, d_status, part.p, ord,
+                                                              stage);
     if (chunks > 1) k_brute_finish<<<fb, 256, 0, s>>>(part.p, nq, d_out);
   } else if (nq < kBruteWarpMaxQueries) {
     // Too few queries for one thread each to fill the GPU (the thread kernel
