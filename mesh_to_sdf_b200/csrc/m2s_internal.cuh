@@ -146,7 +146,7 @@ int drop_pills(DeviceMesh* m, cudaStream_t s);
 // Builds the triangle records and the LBVH.  d_status receives status bits.
 // with_tree = false builds the triangle records only (grid path, brute force).
 int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, cudaStream_t s,
-                      bool with_tree = true);
+                      bool with_tree = true, bool with_pills = true);
 
 // ---- sorting (m2s_sort.cu) ----------------------------------------------------
 

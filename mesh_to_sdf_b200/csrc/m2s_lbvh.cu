@@ -357,7 +357,8 @@ int drop_pills(DeviceMesh* m, cudaStream_t s) {
   return M2S_OK;
 }
 
-int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, cudaStream_t s, bool with_tree) {
+int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, cudaStream_t s, bool with_tree,
+                      bool with_pills) {
   if (in.n_tris > 0x7FFFFFFFull) return M2S_ERR_INVALID_ARGUMENT;
   const uint32_t T = (uint32_t)in.n_tris;
   out->n_tris = T;
@@ -388,7 +389,7 @@ int build_device_mesh(const MeshInput& in, DeviceMesh* out, uint32_t* d_status, 
       (st = counters.alloc(T - 1, s)) || (st = range.alloc(T - 1, s)))
     return st;
   // (pillboxes only make searches faster: a mesh whose tree just fits goes without)
-  if (out->pills.alloc(2ull * (T - 1), s)) cudaGetLastError();
+  if (with_pills && out->pills.alloc(2ull * (T - 1), s)) cudaGetLastError();
   M2S_CUDA(cudaMemsetAsync(counters.p, 0, (T - 1) * sizeof(uint32_t), s));
   k_karras<<<grid_for(T - 1), kThreads, 0, s>>>(keys.p, (int)T, out->nodes.p, node_parent.p, leaf_parent.p,
                                           range.p);
