@@ -913,14 +913,18 @@ struct WarpQueue {
 // k_propagate's block sizes.  An SM holds 1,024 of its threads (64 registers
 // each) as one, two or four blocks.  Fewer blocks are fewer arrivals at a grid
 // barrier and fewer adds to the list counters, more blocks wait less for their
-// slowest warp at block barriers (256 / 512 / 1,024 threads: 32^3 462 / 482 /
-// 515 us, 97 x 110 x 75 2,244 / 2,164 / 2,213, 24 grids of 32M cells 23.2 /
-// 21.7 / 22.2 ms, 256^3 8.69 / 8.48 / 8.32 ms).  The lines lie at the powers
-// of two that bound the autotuner's classes.  blocks_per_sm counts blocks of
-// 256, and the filtered kernel (80 registers) runs three of those per SM.
+// slowest warp at block barriers.  Measured on either side of the lines, 256 / 512 /
+// 1,024 threads in us: star s5 32^3 465 / 469 / 508, 44^3 634 / 605 / 644, 55^3 865 /
+// 801 / 840 (Normal 1,087 / 971 / 986), the terrain 44^3 2,127 / 2,090 / 2,227; star
+// s6 190^3 4,853 / 4,584 / 4,623, 256^3 8,304 / 8,037 / 8,021 (star s3 8,717 / 8,270 /
+// 8,207, s5 Normal 10,168 / 9,724 / 9,663), the terrain 203^3 13,426 / 12,352 / 12,229;
+// batches of 24 grids from 32^3 each (2^19.6 cells) on 512 and 1,024 within 1 %,
+// 80^3 8,274 / 7,940 / 7,881.  The lines are powers of two like the bounds of the
+// autotuner's classes.  blocks_per_sm counts blocks of 256, and the filtered
+// kernel (80 registers) runs three of those per SM.
 constexpr uint32_t kSmallBlock = 256, kBigBlock = 1024;
 inline uint32_t block_threads(unsigned long long cells) {
-  return cells <= 1ull << 18 ? kSmallBlock : (cells <= 1ull << 23 ? 512u : kBigBlock);
+  return cells <= 1ull << 16 ? kSmallBlock : (cells <= 1ull << 23 ? 512u : kBigBlock);
 }
 
 // Stages cell j, whose first lowering of the round this proposal made, for the
@@ -1080,10 +1084,11 @@ __device__ __forceinline__ void relax_commit_solo(const GridSet& gs, unsigned lo
 // the chain.  The pushes leave a copy of each list's first states in shared
 // memory for the next rounds, every warp advances a copy of the schedule of
 // its own instead of waiting for one that does, and only as many warps take
-// part as shorten a typical round.  Rounds of that terrain's grid (Normal), with
+// part as shorten a typical round.  Rounds of one such terrain's grid (Normal), with
 // the whole block at its own barrier before, now: 3.30 -> 2.3 us up to 7
-// states, 3.65 -> 3.2 up to 15; the grid 17.3 -> 15.7 ms (128 / 256 / 512 /
-// 1,024 threads of the run: 16.8 / 15.9 / 15.7 / 16.2).  The schedule's state
+// states, 3.65 -> 3.2 up to 15; that grid 17.3 -> 15.7 ms (128 / 256 / 512 /
+// 1,024 threads of the run: 16.8 / 15.9 / 15.7 / 16.2), others of that size, with
+// more such rounds, 16.9 to 18.9.  The schedule's state
 // leaves the other rounds' registers, which then do not spill for Raycast:
 // 256^3 8.35 -> 8.02 ms, 24 grids of 32M cells 21.5 -> 20.6.  Out of line the
 // run costs the terrain 16.1 ms.
