@@ -153,8 +153,11 @@ int m2s_grid_plan_create(const m2s_mesh* const* meshes, uint32_t n_grids,
 int m2s_grid_plan_run(m2s_grid_plan* plan, void* stream);
 /* Times the plan's waves at several cooperative grid sizes (results are
  * identical at every size) and keeps the fastest per class of wave (device,
- * sign, one grid or several, log2 of the cell count), for this plan and for
- * later plans.  *out_blocks (may be NULL) receives the first wave's choice. */
+ * sign, one grid or several, log2 of the cell count, threads a block), for this
+ * plan and for later plans.  *out_blocks (may be NULL) receives the first wave's
+ * choice, like m2s_grid_plan_blocks in blocks of the wave's own size: 256 threads
+ * up to 2^16 cells, 512 up to 2^23, 1,024 above (256 throughout with
+ * m2s_set_grid_tuning's blocks_per_sm or the filtered variant). */
 int m2s_grid_plan_autotune(m2s_grid_plan* plan, void* stream, uint32_t* out_blocks);
 uint64_t m2s_grid_plan_cells(const m2s_grid_plan* plan);
 uint64_t m2s_grid_plan_device_bytes(const m2s_grid_plan* plan);
@@ -166,8 +169,10 @@ void m2s_grid_plan_free(m2s_grid_plan* plan);
 void m2s_clear_grid_autotune(void);
 
 /* Process-wide grid knobs; they change speed, never results.  blocks_per_sm:
- * cooperative propagation blocks per SM (0 = occupancy limit; the server's
- * grid waves then run 3 per SM, leaving room for point queries);
+ * cooperative propagation blocks of 256 threads per SM (0 = as many threads as
+ * fit, in blocks of 256, 512 or 1,024 by the cell count, the faster shape on
+ * large grids; the server's grid waves then run 2 blocks of 256 per SM, 3 when
+ * alone, leaving room for point queries);
  * cells_per_block: the propagation launch uses ceil(cells / this) blocks, at
  * least one per SM (0 = 1024); wave_cells: a batch runs as jobs of at most this many
  * cells, largest grids first (a larger grid alone); grids in one job share its
@@ -374,8 +379,8 @@ uint32_t m2s_last_grid_round_log(uint32_t* out, uint32_t capacity);
  * (Bvh(Normal): its tie-band fold too).  `node_visits` is the budget of
  * batches of 2^20 queries and more; a batch of nq queries from 2^18 uses
  * node_visits * sqrt(nq / 2^20) and a smaller one node_visits * nq / 2^19, at
- * least 24, since a small batch's time is its longest single-thread search.  0
- * keeps every query on one thread.
+ * least 24 or node_visits, whichever is less, since a small batch's time is its
+ * longest single-thread search.  0 keeps every query on one thread.
  * Process-wide tuning knob; the autotuner sets it. */
 void m2s_set_query_budget(uint32_t node_visits);
 uint32_t m2s_query_budget(void);

@@ -325,11 +325,6 @@ __device__ __forceinline__ TriPlane tri_plane(P3 a, P3 b, P3 c, int kind) {
 __device__ __forceinline__ float plane_query_slack(P3 p) {
   return 0x1p-11f * fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z)));
 }
-// The lower bound of the reference's distance from p (-inf where it does not apply).
-__device__ __forceinline__ float plane_bound(float4 n, float slack, P3 p, float pslack) {
-  const float h = fabsf(fmaf(n.x, p.x, fmaf(n.y, p.y, fmaf(n.z, p.z, -n.w))));
-  return fmaf(h, 1.0f - 0x1p-13f, -(slack + pslack));
-}
 // A bound above this proves the triangle's squared distance exceeds d2.
 __device__ __forceinline__ float plane_above(float d2) { return sqrtf(d2) * (1.0f + 0x1p-18f); }
 

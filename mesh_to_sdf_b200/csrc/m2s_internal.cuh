@@ -174,8 +174,8 @@ int query_points(const MeshView& m, int accel, int sign, const float* d_q, uint6
 // continued one warp per query (0 disables the second pass).
 extern std::atomic<uint32_t> g_query_budget;
 // The budget a batch of nq queries uses: `base` from 2^20 queries up,
-// base * sqrt(nq / 2^20) from 2^18 and base * nq / 2^19 below, at least 24 (0
-// stays 0: no warp pass).  A batch whose queries all have a thread from the
+// base * sqrt(nq / 2^20) from 2^18 and base * nq / 2^19 below, at least
+// min(24, base) (0 stays 0: no warp pass).  A batch whose queries all have a thread from the
 // start waits for its longest searches, which the warp pass finishes sooner;
 // the more queries, the more the thread pass's throughput counts (budgets 24 /
 // 64 / 128 / 192: star s6, RtreeBvh, 20,000 queries 0.35 / 0.39 / 0.43 / 0.45

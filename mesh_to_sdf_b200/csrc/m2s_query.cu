@@ -3,8 +3,9 @@
 //  * None  (generate/generic/default.rs:22-85): k_brute_* — every query against
 //    every triangle.  Triangle tiles are staged in shared memory by the bulk
 //    copy engine (cp.async.bulk + mbarrier, double-buffered); a thread owns two
-//    queries (Raycast) or one (Normal, folded in triangle order, exactly the
-//    reference's fold order); batches of 2^24 pairs or more are visited in Morton order.
+//    queries (Raycast; one against few triangles) or one (Normal, folded in triangle
+//    order, exactly the reference's fold order); batches of 2^24 pairs or more are
+//    visited in Morton order.
 //    Normal batches of fewer than 2^17 queries take k_brute_normal_warp: a
 //    warp per query, the same fold in the same order.
 //  * Bvh(Raycast) / RtreeBvh (bvh.rs:104-180, rtree_bvh.rs:143-201): exact
@@ -544,7 +545,7 @@ __device__ __forceinline__ float pill_dist2(const Pill& pl, P3 p, float ps) {
 // distances where that may prune a search whose best squared distance is `best`
 // (limits: the node's copies of the pillboxes').  The two lie side by side, and
 // both are fetched when either may prune: one trip to memory where one a child
-// made two in a row (star s6: RtreeBvh 1M points 2.40 -> 2.25 ms, 100,000
+// made two in a row (star s6: RtreeBvh 1M points 2.40 -> 2.25 ms in one run, 2.29 to 2.37 over later ones, 100,000
 // Bvh(Normal) 0.69 -> 0.65; terrain 512^2 Rtree 100,000 1.07 -> 1.04, with the
 // order of the leaf tests in walk_lane).
 __device__ __forceinline__ void pill_raise(const Pill* pills, uint32_t node, float limit_l, float limit_r, P3 p, float ps,
