@@ -80,13 +80,32 @@ constexpr int kBfTile = 256;  // triangles per stage: 256 * 48 B = 12 KiB
 // points 0.125 -> 0.082 ms).
 constexpr int kBrThreads = 256;
 constexpr int kBrTile = 64;  // triangles per stage, at most
-// Triangles per stage of a call: fewer where the tiles of 64 would leave SMs
-// idle, since a block's time is its tiles' one after another (1,000 queries on 80 /
-// 320 / 1,280 triangles: tiles of 64 95 / 83 / 78 us, now 29 / 30 / 33).
-inline uint32_t brute_tile(uint32_t n_tris, uint32_t blocks) {
-  uint32_t tile = kBrTile;
-  while (tile > 8 && (uint64_t)blocks * ((n_tris + tile - 1) / tile) < 2 * 148) tile /= 2;
-  return tile;
+// How a call's triangles are split: stages of `stage` triangles, `chunks` of them
+// to as many blocks for each block of queries.
+//  * Stages are shorter where those of 64 would leave SMs idle, since a block's
+//    time is its stages' one after another (1,000 queries on 80 / 320 / 1,280
+//    triangles: stages of 64 95 / 83 / 78 us, now 29 / 30 / 33).
+//  * Blocks that fill the GPU once to four times (four an SM) are made as many as
+//    fit at once, since the few of a last turn took as long as a full one (terrain,
+//    queries x triangles: 4,500 x 4,602 208 -> 171 us, 3,000 x 8,186 222 -> 190,
+//    1,024 x 19,994 245 -> 154, 1,287 x 44,994 465 -> 416; star 2,000 x 20,480 200 -> 175).
+struct BruteSplit {
+  uint32_t stage, chunks;
+};
+inline BruteSplit brute_split(uint32_t n_tris, uint32_t blocks) {
+  constexpr uint32_t kTurn = 148 * 4;
+  auto count = [&](uint32_t per) { return (n_tris + per - 1) / per; };
+  uint32_t stage = kBrTile;
+  while (stage > 8 && (uint64_t)blocks * count(stage) < 2 * 148) stage /= 2;
+  const uint64_t all = (uint64_t)blocks * count(kBrTile);
+  if (all > kTurn && all <= 4 * kTurn && blocks <= kTurn) {
+    const uint32_t per = count(kTurn / blocks);  // triangles of a chunk
+    const uint32_t stages = (per + kBrTile - 1) / kBrTile;
+    return {(per + stages - 1) / stages, kTurn / blocks};
+  }
+  // Enough (query, triangle chunk) blocks to fill the GPU ~4 deep.
+  const uint32_t chunks = (uint32_t)std::max<uint64_t>(1, (148ull * 16ull + blocks - 1) / blocks);
+  return {stage, std::max(1u, std::min(chunks, std::min(count(stage), 256u)))};
 }
 
 typedef unsigned long long f32x2;
@@ -150,7 +169,7 @@ __global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* _
   }
   const f32x2 px = pack2(p[0].x, p[1].x), py = pack2(p[0].y, p[1].y), pz = pack2(p[0].z, p[1].z);
   // this block's chunk of triangles: whole tiles [t_begin, t_end)
-  const uint32_t all_tiles = (T + stage - 1) / stage;  // stage: brute_tile
+  const uint32_t all_tiles = (T + stage - 1) / stage;  // stage: brute_split
   const uint32_t per = (all_tiles + gridDim.y - 1) / gridDim.y;
   const uint32_t t_begin = min(all_tiles, blockIdx.y * per), t_end = min(all_tiles, t_begin + per);
   const uint32_t ntile = t_end - t_begin;
@@ -314,7 +333,7 @@ __global__ void __launch_bounds__(kBrThreads, 4) k_brute_raycast(const TriRec* _
 // and a chain of distances set the time, so there is nothing to split or to skip,
 // and the closest point is the one without branches (a warp's queries lie in
 // different regions).  In us, one query a thread with planes (the kernel before the
-// packed one) / packed with tiles of 64 / packed with brute_tile / this one: 20
+// packed one) / packed with tiles of 64 / packed with brute_split / this one: 20
 // triangles, 1,000 queries 26 / 45 / 34 / 22; 44, 100,000 50 / 78 / 73 / 42; 80,
 // 30,000 56 / 98 / 45 / 52, 100,000 82 / 123 / 119 / 75, 500,000 316 / 230 / 230 / 310;
 // 194, 50,000 115 / 124 / 123 / 111, 200,000 282 / 258 / 257 / 285.
@@ -429,7 +448,11 @@ __global__ void k_brute_finish(const uint2* __restrict__ part, uint64_t nq, floa
 // groups then need no compare_distances at all.
 constexpr int kBwThreads = 256;                 // 8 queries per block
 constexpr uint64_t kBruteWarpMaxQueries = 1u << 17;  // below: one warp per query
-constexpr uint64_t kBruteSortMinPairs = 1ull << 24;  // from here the thread kernels visit queries in Morton order
+// Pairs from which the thread kernels visit queries in Morton order.  A few thousand
+// queries lie too far apart for their order to help as much: 1,300 to 3,000 points on
+// terrain, 2^24 to 2^25 pairs, took 10 to 40 us longer ordered (1,287 x 16,194 228 us, 203),
+// 16,000 on 1,280 triangles 171 us against 145.
+inline uint64_t brute_sort_min_pairs(uint64_t nq) { return nq < 8192 ? 1ull << 25 : 1ull << 24; }
 __global__ void __launch_bounds__(kBwThreads) k_brute_normal_warp(const TriRec* __restrict__ tris, uint32_t T,
                                                                   const float* __restrict__ q, uint64_t nq,
                                                                   float* __restrict__ out, uint32_t* status) {
@@ -1588,8 +1611,8 @@ __global__ void k_bf_keys(const float* __restrict__ q, uint64_t nq, const int* _
 int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, float* d_out, uint32_t* d_status,
                     cudaStream_t s, bool allow_alloc) {
   if (nq == 0) return M2S_OK;
-  // Thread-per-query kernels visit batches of 2^24 pairs or more, at least
-  // 1,024 queries, in Morton order (of the queries' own bounding box): the
+  // Thread-per-query kernels visit batches of many pairs (brute_sort_min_pairs), at
+  // least 1,024 queries, in Morton order (of the queries' own bounding box): the
   // lanes of a warp then mostly agree on which planes come near and fall in
   // the same Voronoi regions (Raycast, 10,000 points x 20,480 triangles 0.82
   // -> 0.52 ms; the sort takes about 0.05 ms).  Results are per query, so the
@@ -1599,7 +1622,7 @@ int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, 
   const uint32_t* ord = nullptr;
   const bool few = sign == M2S_SIGN_RAYCAST && brute_few(m.n_tris, nq);
   const bool thread_kernel = !few && (sign == M2S_SIGN_RAYCAST || nq >= kBruteWarpMaxQueries);
-  if (allow_alloc && thread_kernel && nq >= 1024 && nq <= 0xFFFFFFFFull && nq * m.n_tris >= kBruteSortMinPairs) {
+  if (allow_alloc && thread_kernel && nq >= 1024 && nq <= 0xFFFFFFFFull && nq * m.n_tris >= brute_sort_min_pairs(nq)) {
     int st;
     if ((st = keys.alloc(nq, s)) || (st = order.alloc(nq, s)) || (st = bounds.alloc(6, s))) return st;
     k_bf_bounds_init<<<1, 32, 0, s>>>(bounds.p);
@@ -1612,11 +1635,8 @@ int brute_force_sdf(const MeshView& m, int sign, const float* d_q, uint64_t nq, 
   if (few) {
     k_brute_raycast_few<<<(unsigned)((nq + 127) / 128), 128, 0, s>>>(m.tris, m.n_tris, d_q, nq, d_out);
   } else if (sign == M2S_SIGN_RAYCAST) {
-    // Enough (query, triangle chunk) blocks to fill the GPU ~4 deep.
     const unsigned blocks = (unsigned)((nq + 2 * kBrThreads - 1) / (2 * kBrThreads));
-    const uint32_t stage = brute_tile(m.n_tris, blocks), tiles = (m.n_tris + stage - 1) / stage;
-    uint32_t chunks = (uint32_t)std::max<uint64_t>(1, (148ull * 16ull + blocks - 1) / blocks);
-    chunks = std::max(1u, std::min(chunks, std::min(tiles, 256u)));
+    const auto [stage, chunks] = brute_split(m.n_tris, blocks);
     DevBuf<uint2> part;
     int st;
     if (chunks > 1 && allow_alloc && (st = part.alloc(nq, s))) return st;

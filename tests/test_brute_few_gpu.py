@@ -24,3 +24,15 @@ def test_small_meshes(orc, tris, n):
     got = m2s.generate_sdf(v, m2s.Topology.TriangleList(keep), q, AM)
     exp = orc.generate_sdf(v, keep, q, "none", "raycast")
     assert np.array_equal(got.view(np.uint32), exp.view(np.uint32))
+
+
+# blocks of queries and tiles that just fill the GPU (592 blocks), fill it a little more than once and four times
+@pytest.mark.parametrize("tris,n", [(4602, 4500), (4602, 4097), (8186, 3000), (19994, 1024), (19994, 7000), (1280, 60000),
+                                    (300, 303105)])
+def test_blocks_that_fit_at_once(orc, tris, n):
+    v, idx = synth.star(5, seed=9)
+    keep = idx[:3 * tris]
+    q = synth.mixed_points(v, idx, n, seed=n % 997)
+    got = m2s.generate_sdf(v, m2s.Topology.TriangleList(keep), q, AM)
+    exp = orc.generate_sdf(v, keep, q, "none", "raycast")
+    assert np.array_equal(got.view(np.uint32), exp.view(np.uint32))
