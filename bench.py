@@ -36,7 +36,7 @@ SEED = 0
 
 # DRAM bytes (read + write) of one propagation launch of the bench grid, from
 # an ncu capture of dram__bytes_read.sum and dram__bytes_write.sum (one launch).
-PROPAGATE_DRAM_BYTES = 145_844_224 + 243_579_392
+PROPAGATE_DRAM_BYTES = 145_277_952 + 241_163_520
 PROPAGATE_DRAM_SOURCE = "profiles/k_propagate_star_s6_grid256.md (ncu, one 256^3 launch)"
 
 
@@ -555,6 +555,7 @@ def main():
     # step; results are identical), and the FP64 audit of the grid's f32
     # decisions (counts only)
     m2s.set_grid_bound_filter(True)
+    step()  # loads the variant's kernel
     m2s.set_profiling(True)
     flush.fill_(1)
     step()
