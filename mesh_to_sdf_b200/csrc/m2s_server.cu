@@ -32,8 +32,8 @@
 // what the budget has to spare: no request is refused, delayed behind idle
 // memory or answered by an eviction because of them.  They are counted beside
 // the reservations, and when a reservation needs their room, meshes that no
-// request runs on give theirs back, least recently used first; those that one
-// runs on are waited for.
+// request runs on give theirs back, least recently used first.  Where that is not
+// enough, meshes that one runs on take no further request until theirs are given back.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -90,6 +90,7 @@ struct MeshEntry {
   int users = 0;  // queued or running requests
   int running = 0;  // running ones
   uint64_t pills = 0;  // bytes of its pillboxes, in m2s_server::spare
+  bool drain = false;  // no request starts on it until the running ones are done and its pillboxes given back
   bool failed = false;
 };
 
@@ -163,15 +164,35 @@ struct m2s_server {
 
   // ---- helpers (mu held) ----
   bool fits(uint64_t need) const { return reserved + need <= budget; }
-  // `need` fits beside the pillboxes that running requests read.
-  bool admits(uint64_t need) const { return reserved + need + busy <= budget; }
+  // `need` fits beside the pillboxes that running requests read.  Where only these
+  // are in the way, enough of them are marked to be given back, so that a mesh
+  // that is never idle does not keep the request waiting.
+  bool admits(uint64_t need) {
+    if (!fits(need)) return false;
+    const uint64_t most = budget - reserved - need;  // room for pillboxes
+    if (busy <= most) return true;
+    uint64_t kept = busy;
+    for (auto& kv : meshes)
+      if (kv.second.drain) kept -= kv.second.pills;
+    while (kept > most) {
+      MeshEntry* victim = nullptr;
+      for (auto& kv : meshes)
+        if (kv.second.running && kv.second.pills && !kv.second.drain &&
+            (!victim || kv.second.last_use < victim->last_use))
+          victim = &kv.second;
+      if (!victim) break;
+      victim->drain = true;
+      kept -= victim->pills;
+    }
+    return false;
+  }
   // The head of queue k can be taken now: its mesh is gone or failed (it
   // completes with an error), or its mesh is resident and it fits.
-  bool head_ready(int k) const {
+  bool head_ready(int k) {
     if (q[k].empty()) return false;
     const RequestP& r = q[k].front();
     auto it = meshes.find(r->mesh_id);
-    return it == meshes.end() || it->second.failed || (it->second.mesh && admits(r->need));
+    return it == meshes.end() || it->second.failed || (it->second.mesh && !it->second.drain && admits(r->need));
   }
   void reserve(uint64_t need) {
     reserved += need;
@@ -180,12 +201,16 @@ struct m2s_server {
       for (auto& kv : meshes)
         if (kv.second.pills && !kv.second.running && (!victim || kv.second.last_use < victim->last_use))
           victim = &kv.second;
-      // (no search reads them: no request runs on the mesh)
-      if (!victim || drop_pills(&victim->mesh->mesh, s_trim)) break;
-      spare -= victim->pills;
-      victim->pills = 0;
+      if (!victim || !give_back(*victim)) break;
     }
     peak = std::max(peak, reserved + spare);
+  }
+  // The pillboxes of a mesh that no request runs on (so no search reads them).
+  bool give_back(MeshEntry& e) {
+    if (e.pills && drop_pills(&e.mesh->mesh, s_trim)) return false;
+    spare -= e.pills;
+    e.pills = 0;
+    return true;
   }
   // A request leaves its queue for the mesh it needs.
   void start(const RequestP& r, MeshEntry& e) {
@@ -203,7 +228,11 @@ struct m2s_server {
       auto it = meshes.find(r->mesh_id);
       if (it != meshes.end()) {
         it->second.users--;
-        if (r->running && --it->second.running == 0) busy -= it->second.pills;
+        if (r->running && --it->second.running == 0) {
+          busy -= it->second.pills;
+          if (it->second.drain) give_back(it->second);
+          it->second.drain = false;
+        }
       }
     }
     if (status == M2S_OK) completed[r->kind]++;
@@ -324,7 +353,7 @@ void m2s_server::points_loop() {
           finish(r, M2S_ERR_INVALID_ARGUMENT);
           continue;
         }
-        if (!it->second.mesh || !admits(r->need)) break;
+        if (!it->second.mesh || it->second.drain || !admits(r->need)) break;
         q[kPoints].pop_front();
         start(r, it->second);
         go.emplace_back(r, it->second.mesh);
@@ -424,7 +453,7 @@ void m2s_server::grid_loop(int lane) {
           finish(r, M2S_ERR_INVALID_ARGUMENT);
           continue;
         }
-        if (!it->second.mesh || !admits(r->need)) break;
+        if (!it->second.mesh || it->second.drain || !admits(r->need)) break;
         if (!wave.empty() && r->grid_sign != wave.front()->grid_sign) break;  // one sign per wave
         if (!wave.empty() && cells + r->cells > tune.wave_cells) break;
         q[kGrid].pop_front();

@@ -85,3 +85,34 @@ def test_several_meshes(extra):
             assert st["reserved_bytes"] == held + 3 * 64 * (tris - 1)
     finally:
         srv.close()
+
+
+def test_upload_beside_a_busy_mesh():
+    """An upload that only the pillboxes of a mesh with a stream of requests are in the way of."""
+    (v, idx), (v2, idx2) = synth.star(4, seed=7), synth.star(4, seed=8)
+    lo, hi = synth.padded_bbox(v)
+    q = synth.uniform_points(60000, lo, hi, seed=3)
+    tris, point = len(idx) // 3, 64 * len(q) + MB
+    budget = 160 * tris + 2 * point + upload_need(v2, idx2) + 100_000  # less than the pillboxes' 327,616
+    srv = m2s.Server(budget)
+    try:
+        mid, t = srv.submit_upload(v, T.TriangleList(idx), A.rtree_bvh())
+        assert srv.wait(t, timeout_s=60)[0] == 0
+        outs = [np.empty(len(q), np.float32) for _ in range(40)]
+        jobs = [srv.submit_points(mid, q, o) for o in outs[:20]]
+        mid2, t2 = srv.submit_upload(v2, T.TriangleList(idx2), A.rtree_bvh())
+        jobs += [srv.submit_points(mid, q, o) for o in outs[20:]]
+        assert srv.wait(t2, timeout_s=60)[0] == 0
+        last = np.empty(1000, np.float32)
+        jobs.append(srv.submit_points(mid2, q[:1000], last))
+        for t in jobs:
+            assert srv.wait(t, timeout_s=60)[0] == 0
+        ref = m2s.query_sdf(m2s.build_sdf_acceleration(v, T.TriangleList(idx), A.rtree_bvh()), q)
+        for o in outs:
+            assert np.array_equal(bits(o), bits(ref))
+        ref2 = m2s.query_sdf(m2s.build_sdf_acceleration(v2, T.TriangleList(idx2), A.rtree_bvh()), q[:1000])
+        assert np.array_equal(bits(last), bits(ref2))
+        st = srv.stats()
+        assert st["failed"] == 0 and st["evictions"] == 0 and st["queued"] == 0 and st["reserved_bytes"] <= budget
+    finally:
+        srv.close()
