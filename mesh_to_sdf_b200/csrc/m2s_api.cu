@@ -324,10 +324,14 @@ int m2s_generate_sdf(const float* vertices, uint64_t nv, const void* indices, ui
   cudaStream_t s = (cudaStream_t)stream;
   m2s_mesh h;
   // Pillboxes cost a build 20 us and about 0.2 us per 1,000 triangles, which a few
-  // queries do not earn back: 100 queries on 524,282 triangles of terrain 1,143 us a
-  // call with them, 1,001 without (1,060 before there were any), on 81,920 of the star
-  // 529 either way; from 2,000 queries on the terrain they cost 3 to 8 % of a call.
-  const bool with_pills = nq >= T / 512;
+  // queries do not earn back (us a call without / with them, before there were any):
+  // 100 queries on 524,282 triangles of terrain 1,001 / 1,143, 1,060, on 81,920 of the
+  // star 529 / 529, 602; 1,000 on 320, 1,280 and 5,120 181 / 192, 203; 209 / 221, 248;
+  // 288 / 275, 330; 300 on 20,480 367 / 338, 440.  Bvh(Normal), which walks the tree
+  // twice, earns them back sooner: 100 on 81,920 593 / 512, 670, 300 on 5,120 278 /
+  // 260, 317.  From 2,000 queries on that terrain they cost 3 to 8 % of a call.
+  const bool twice = accel == M2S_ACCEL_BVH && sign == M2S_SIGN_NORMAL;
+  const bool with_pills = nq >= T / (twice ? 1024 : 512) && nq * T >= 1ull << (twice ? 20 : 22);
   if ((st = build_mesh_handle(vertices, nv, indices, ni, bits, topo, accel, sign, T, &h, s, with_pills))) {
     // generate_sdf_default never reads a vertex when there is no query.
     if (!(st == M2S_ERR_INDEX_RANGE && accel == M2S_ACCEL_NONE && nq == 0)) return st;

@@ -1,4 +1,5 @@
-"""generate_sdf around the number of queries from which its tree gets pillboxes (one per 512 triangles), bit for bit."""
+"""generate_sdf around the number of queries from which its tree gets pillboxes (one per 512
+triangles and 2^22 pairs, for Bvh(Normal) one per 1,024 and 2^20), bit for bit."""
 import numpy as np
 import pytest
 
@@ -9,7 +10,7 @@ pytestmark = pytest.mark.gpu
 A, S = m2s.AccelerationMethod, m2s.SignMethod
 
 
-@pytest.mark.parametrize("n", [1, 9, 10, 39, 40, 41])  # 5,120 and 20,480 triangles
+@pytest.mark.parametrize("n", [1, 51, 52, 204, 205, 819, 820])  # 5,120 and 20,480 triangles
 @pytest.mark.parametrize("subdiv", [4, 5])
 def test_few_queries(orc, subdiv, n):
     v, idx = synth.star(subdiv, seed=6)
