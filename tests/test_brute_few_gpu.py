@@ -21,6 +21,8 @@ def test_small_meshes(orc, tris, n):
     keep = keep.reshape(-1)
     q = synth.mixed_points(v, idx, n, seed=n % 997)
     q[0] = v[keep[0]]
+    far = np.array([[1e30, 0, 0], [-3e19, 1e19, 0], [1e-30, 0, 1e-38], [2e38, 2e38, 2e38]], np.float32)
+    q[1:5] = far[:max(0, min(4, n - 1))]  # squares overflow; denormal
     got = m2s.generate_sdf(v, m2s.Topology.TriangleList(keep), q, AM)
     exp = orc.generate_sdf(v, keep, q, "none", "raycast")
     assert np.array_equal(got.view(np.uint32), exp.view(np.uint32))
